@@ -240,6 +240,47 @@ void dfree(void*& p) {
   p = nullptr;
 }
 
+// One device allocation for the temporaries of a call, each piece on a
+// 256-byte boundary, given back when the object goes out of scope.  Not
+// zero-filled: every piece is written before it is read, in stream order.
+// (A call that took each piece with dmalloc paid a cudaMalloc, a cleared copy
+// of the piece, a synchronisation and a cudaFree for every one of them.)
+struct Scratch {
+  unsigned char* base = nullptr;
+  size_t bytes = 0;
+  size_t take(size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) & ~(size_t)255;
+    return at;
+  }
+  int alloc(std::string* errp) {
+    CK(cudaMalloc((void**)&base, bytes ? bytes : 256));
+    return MRM_OK;
+  }
+  template <typename T>
+  T* at(size_t off) const { return reinterpret_cast<T*>(base + off); }
+  Scratch() = default;
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  ~Scratch() {
+    if (base) cudaFree(base);
+  }
+};
+
+// FP64 twiddles of kTwN points (an engine's table may be FP32)
+const std::vector<double>& twiddles64() {
+  static const std::vector<double> tw = [] {
+    std::vector<double> v(2 * kTwN);
+    for (int k = 0; k < kTwN; ++k) {
+      const double a = -2.0 * M_PI * (double)k / (double)kTwN;
+      v[2 * k] = std::cos(a);
+      v[2 * k + 1] = std::sin(a);
+    }
+    return v;
+  }();
+  return tw;
+}
+
 struct CudaFreeDeleter {
   void operator()(void* p) const {
     if (p) cudaFree(p);
@@ -1729,27 +1770,45 @@ std::vector<PairGeom> pair_geoms(const mrm_gpu* r) {
   return out;
 }
 
-// real-space FP64 tensor on the device (reference layout)
-int tensor_real(mrm_gpu* r, double* d_n2d) {
+cudaError_t launch_tensor_real(double* d_n2d, const PairGeom* d_pg, int npair, int px, int py, double dx, double dy,
+                               int nimg, cudaStream_t st) {
+  const size_t smem = tens_smem(dx == dy);
+  const cudaError_t ce = allow_smem((const void*)tensor_real_kernel, smem);
+  if (ce != cudaSuccess) return ce;
+  const unsigned tiles = (unsigned)(((px / 2 + kTensTile) / kTensTile) * ((py / 2 + kTensTile) / kTensTile));
+  tensor_real_kernel<<<dim3(tiles, npair), kTensBlock, smem, st>>>(d_n2d, d_pg, px, py, dx, dy, nimg);
+  return cudaGetLastError();
+}
+
+// Temporaries of a tensor build: the real tensor, its spectrum, FP64
+// twiddles, the pair geometries and the two diagnostic maxima.
+struct TensorScratch : Scratch {
+  size_t n2d, spec, tw, pg, mx;
+  TensorScratch(const mrm_gpu* r, bool spectrum) {
+    const size_t npair = (size_t)r->nl * r->nl, planes = npair * 9;
+    n2d = take(sizeof(double) * planes * r->px * r->py);
+    pg = take(sizeof(PairGeom) * npair);
+    mx = take(2 * sizeof(unsigned long long));
+    spec = spectrum ? take(sizeof(double) * 2 * planes * r->py * (r->px / 2 + 1)) : 0;
+    tw = spectrum ? take(sizeof(double) * 2 * kTwN) : 0;
+  }
+};
+
+// real-space FP64 tensor on the device (reference layout), enqueued on the
+// engine's stream
+int tensor_real(mrm_gpu* r, const TensorScratch& w) {
   std::string* errp = &r->err;
   const int npair = r->nl * r->nl;
-  std::vector<PairGeom> pg = pair_geoms(r);
-  void* d_pg = nullptr;
-  int rc = dmalloc(errp, &d_pg, sizeof(PairGeom) * npair);
-  if (rc) return rc;
-  CK(h2d(d_pg, pg.data(), sizeof(PairGeom) * npair));
+  const std::vector<PairGeom> pg = pair_geoms(r);
+  CK(h2d(w.at<PairGeom>(w.pg), pg.data(), sizeof(PairGeom) * npair));
   const int nimg = r->g.boundary == MRM_OPEN ? 0 : std::max(0, r->g.num_images);
-  const long long total = (long long)npair * r->px * r->py;
-  tensor_real_kernel<<<(unsigned)((total + 127) / 128), 128, 0, r->eng->st>>>(
-      d_n2d, static_cast<const PairGeom*>(d_pg), npair, r->px, r->py, r->g.dx, r->g.dy, nimg);
-  CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(r->eng->st));
-  dfree(d_pg);
+  CK(launch_tensor_real(w.at<double>(w.n2d), w.at<PairGeom>(w.pg), npair, r->px, r->py, r->g.dx, r->g.dy, nimg,
+                        r->eng->st));
   return MRM_OK;
 }
 
 // FP64 FFT of the real tensor and packing into the run's spectral store
-int tensor_spectrum(mrm_gpu* r, const double* d_n2d) {
+int tensor_spectrum(mrm_gpu* r, const TensorScratch& w) {
   std::string* errp = &r->err;
   Engine* e = r->eng;
   // a buffer shared with other runs is left to them: this run writes its own
@@ -1760,45 +1819,33 @@ int tensor_spectrum(mrm_gpu* r, const double* d_n2d) {
   }
   const int npair = r->nl * r->nl, ph = r->px / 2 + 1, pyh = r->py / 2 + 1;
   const int planes = npair * 9;
-  void* d_spec = nullptr;
-  int rc = dmalloc(errp, &d_spec, sizeof(double) * 2 * (size_t)planes * r->py * ph);
-  if (rc) return rc;
-  // FP64 twiddles (the engine's table may be FP32)
-  void* d_tw64 = nullptr;
-  std::vector<double> tw(2 * kTwN);
-  for (int k = 0; k < kTwN; ++k) {
-    double a = -2.0 * M_PI * (double)k / (double)kTwN;
-    tw[2 * k] = std::cos(a);
-    tw[2 * k + 1] = std::sin(a);
-  }
-  rc = dmalloc(errp, &d_tw64, sizeof(double) * 2 * kTwN);
-  if (rc) return rc;
-  CK(h2d(d_tw64, tw.data(), sizeof(double) * 2 * kTwN));
-  const Cx<double>* tw64 = static_cast<const Cx<double>*>(d_tw64);
+  const double* d_n2d = w.at<double>(w.n2d);
+  Cx<double>* d_spec = w.at<Cx<double>>(w.spec);
+  const Cx<double>* tw64 = w.at<Cx<double>>(w.tw);
+  unsigned long long* d_mx = w.at<unsigned long long>(w.mx);
+  CK(h2d(w.at<double>(w.tw), twiddles64().data(), sizeof(double) * 2 * kTwN));
+  CK(cudaMemsetAsync(d_mx, 0, 2 * sizeof(unsigned long long), e->st));
   const int M = r->px / 2;
   // two shared buffers of one padded-stride sequence each (fft.cuh)
   size_t s1 = 2 * (size_t)pad_stride(M) * sizeof(Cx<double>), s2 = 2 * (size_t)pad_stride(r->py) * sizeof(Cx<double>);
   CK(allow_smem((const void*)r2c_rows_f64, s1));
   CK(allow_smem((const void*)c2c_cols_f64, s2));
-  r2c_rows_f64<<<planes * r->py, 256, s1, e->st>>>(d_n2d, static_cast<Cx<double>*>(d_spec), r->lgpx, r->py, tw64);
+  r2c_rows_f64<<<planes * r->py, 256, s1, e->st>>>(d_n2d, d_spec, r->lgpx, r->py, tw64);
   CK(cudaGetLastError());
-  c2c_cols_f64<<<planes * ph, 256, s2, e->st>>>(static_cast<Cx<double>*>(d_spec), r->lgpy, ph, tw64);
+  c2c_cols_f64<<<planes * ph, 256, s2, e->st>>>(d_spec, r->lgpy, ph, tw64);
   CK(cudaGetLastError());
-  unsigned long long* d_mx = nullptr;
-  rc = dmalloc(errp, (void**)&d_mx, 2 * sizeof(unsigned long long));
-  if (rc) return rc;
   if (e->prec == MRM_FP64) {
     const long long total = (long long)ph * npair * 9 * r->py;
     pack_tensor_full_kernel<<<(unsigned)((total + 255) / 256), 256, 0, e->st>>>(
-        static_cast<const Cx<double>*>(d_spec), static_cast<Cx<double>*>(r->tens), npair, r->py, ph, d_mx, d_mx + 1);
+        d_spec, static_cast<Cx<double>*>(r->tens), npair, r->py, ph, d_mx, d_mx + 1);
   } else if (creg_run(r)) {
     const long long total = (long long)ph * 6 * r->py;
     pack_tensor_creg_kernel<<<(unsigned)((total + 255) / 256), 256, 0, e->st>>>(
-        static_cast<const Cx<double>*>(d_spec), static_cast<float*>(r->tens), r->lgpy, ph, d_mx, d_mx + 1);
+        d_spec, static_cast<float*>(r->tens), r->lgpy, ph, d_mx, d_mx + 1);
   } else {
     const long long total = (long long)ph * npair * 9 * pyh;
     pack_tensor_kernel<float><<<(unsigned)((total + 255) / 256), 256, 0, e->st>>>(
-        static_cast<const Cx<double>*>(d_spec), static_cast<float*>(r->tens), npair, r->py, ph,
+        d_spec, static_cast<float*>(r->tens), npair, r->py, ph,
         tens_row_stride(r->py), d_mx, d_mx + 1);
   }
   CK(cudaGetLastError());
@@ -1810,12 +1857,10 @@ int tensor_spectrum(mrm_gpu* r, const double* d_n2d) {
   std::memcpy(&dkept, &hm[1], 8);
   r->tensor_resid = dres;
   r->tensor_kept = dkept;
-  dfree(d_mx);
-  dfree(d_spec);
-  dfree(d_tw64);
+  // (the tasks list the runs with a tensor: a rebuilt one changes none of them)
+  if (!r->tensor_ready) e->tables_dirty = true;
   r->tensor_ready = true;
   r->spec_valid = false;
-  e->tables_dirty = true;
   e->desc_dirty = true;
   return MRM_OK;
 }
@@ -2051,40 +2096,29 @@ int mrm_gpu_off_field(mrm_gpu* h, double zoff, double dzobs, double head_mu, dou
   }
   const int ph = nx / 2 + 1, lgx = ilog2(nx), lgy = ilog2(ny);
   const size_t plane = (size_t)nx * ny, hplane = (size_t)ph * ny;
-  void *d_pg = nullptr, *d_t = nullptr, *d_ts = nullptr, *d_m = nullptr, *d_ms = nullptr, *d_h = nullptr,
-       *d_out = nullptr, *d_tw = nullptr;
+  Scratch w;
+  const size_t o_pg = w.take(sizeof(PairGeom) * nl), o_t = w.take(sizeof(double) * 9 * nl * plane),
+               o_ts = w.take(sizeof(double) * 2 * 9 * nl * hplane), o_m = w.take(sizeof(double) * 3 * nl * plane),
+               o_ms = w.take(sizeof(double) * 2 * 3 * nl * hplane), o_h = w.take(sizeof(double) * 2 * 3 * hplane),
+               o_out = w.take(sizeof(double) * 3 * plane), o_tw = w.take(sizeof(double) * 2 * kTwN);
+  rc = w.alloc(errp);
+  if (rc) return rc;
+  void *d_pg = w.at<void>(o_pg), *d_t = w.at<void>(o_t), *d_ts = w.at<void>(o_ts), *d_m = w.at<void>(o_m),
+       *d_ms = w.at<void>(o_ms), *d_h = w.at<void>(o_h), *d_out = w.at<void>(o_out), *d_tw = w.at<void>(o_tw);
+  // (a failure waits for what is in flight on the temporaries)
   auto finish = [&](int code) {
-    for (void* q : {d_pg, d_t, d_ts, d_m, d_ms, d_h, d_out, d_tw}) {
-      void* qq = q;
-      dfree(qq);
-    }
+    if (code) cudaStreamSynchronize(e->st);
     return code;
   };
-  rc = dmalloc(errp, &d_pg, sizeof(PairGeom) * nl);
-  if (!rc) rc = dmalloc(errp, &d_t, sizeof(double) * 9 * nl * plane);
-  if (!rc) rc = dmalloc(errp, &d_ts, sizeof(double) * 2 * 9 * nl * hplane);
-  if (!rc) rc = dmalloc(errp, &d_m, sizeof(double) * 3 * nl * plane);
-  if (!rc) rc = dmalloc(errp, &d_ms, sizeof(double) * 2 * 3 * nl * hplane);
-  if (!rc) rc = dmalloc(errp, &d_h, sizeof(double) * 2 * 3 * hplane);
-  if (!rc) rc = dmalloc(errp, &d_out, sizeof(double) * 3 * plane);
-  if (!rc) rc = dmalloc(errp, &d_tw, sizeof(double) * 2 * kTwN);
-  if (rc) return finish(rc);
-  std::vector<double> tw(2 * kTwN);
-  for (int k = 0; k < kTwN; ++k) {
-    const double a = -2.0 * M_PI * (double)k / (double)kTwN;
-    tw[2 * k] = std::cos(a);
-    tw[2 * k + 1] = std::sin(a);
-  }
   const cudaStream_t st = e->st;
   auto ok = [&](cudaError_t c) { return c == cudaSuccess; };
-  if (!ok(cudaMemcpyAsync(d_tw, tw.data(), sizeof(double) * 2 * kTwN, cudaMemcpyHostToDevice, st)) ||
+  if (!ok(cudaMemcpyAsync(d_tw, twiddles64().data(), sizeof(double) * 2 * kTwN, cudaMemcpyHostToDevice, st)) ||
       !ok(cudaMemcpyAsync(d_pg, pg.data(), sizeof(PairGeom) * nl, cudaMemcpyHostToDevice, st)))
     return finish(set_err(errp, MRM_ERR_CUDA, "off-plane field: copy"));
   const Cx<double>* tw64 = static_cast<const Cx<double>*>(d_tw);
-  const long long tot = (long long)nl * plane;
-  tensor_real_kernel<<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(static_cast<double*>(d_t),
-                                                                     static_cast<const PairGeom*>(d_pg), nl, nx, ny,
-                                                                     g.dx, g.dy, num_images);
+  if (!ok(launch_tensor_real(static_cast<double*>(d_t), static_cast<const PairGeom*>(d_pg), nl, nx, ny, g.dx, g.dy,
+                             num_images, st)))
+    return finish(set_err(errp, MRM_ERR_CUDA, "off-plane field: tensor"));
   if (e->prec == MRM_FP64)
     mgrid_kernel<double><<<dim3((unsigned)((plane + 255) / 256), nl), 256, 0, st>>>(
         static_cast<const RunDev<double>*>(e->d_runs), h->slot, static_cast<double*>(d_m));
@@ -2122,13 +2156,10 @@ int mrm_gpu_build_tensor(mrm_gpu* h) {
   std::string* errp = &h->err;
   if (int rc = need_fft(h)) return rc;
   CK(cudaSetDevice(h->eng->dev));
-  void* d_n2d = nullptr;
-  const size_t bytes = sizeof(double) * 9 * (size_t)h->nl * h->nl * h->px * h->py;
-  int rc = dmalloc(errp, &d_n2d, bytes);
-  if (rc) return rc;
-  rc = tensor_real(h, static_cast<double*>(d_n2d));
-  if (!rc) rc = tensor_spectrum(h, static_cast<const double*>(d_n2d));
-  dfree(d_n2d);
+  TensorScratch w(h, true);
+  int rc = w.alloc(errp);
+  if (!rc) rc = tensor_real(h, w);
+  if (!rc) rc = tensor_spectrum(h, w);
   return rc;
 }
 
@@ -2139,31 +2170,24 @@ int mrm_gpu_upload_tensor(mrm_gpu* h, const double* n2d, int nx_fft, int ny_fft)
   if (nx_fft != h->px || ny_fft != h->py)
     return set_err(errp, MRM_ERR_ARG, "tensor grid %dx%d differs from the FFT grid %dx%d", nx_fft, ny_fft, h->px, h->py);
   CK(cudaSetDevice(h->eng->dev));
-  void* d_n2d = nullptr;
-  const size_t bytes = sizeof(double) * 9 * (size_t)h->nl * h->nl * h->px * h->py;
-  int rc = dmalloc(errp, &d_n2d, bytes);
-  if (rc) return rc;
-  CK(h2d(d_n2d, n2d, bytes));
-  rc = tensor_spectrum(h, static_cast<const double*>(d_n2d));
-  dfree(d_n2d);
-  return rc;
+  TensorScratch w(h, true);
+  if (int rc = w.alloc(errp)) return rc;
+  CK(h2d(w.at<double>(w.n2d), n2d, sizeof(double) * 9 * (size_t)h->nl * h->nl * h->px * h->py));
+  return tensor_spectrum(h, w);
 }
 
 int mrm_gpu_download_tensor(mrm_gpu* h, double* n2d) {
   if (!h || !n2d) return MRM_ERR_ARG;
   std::string* errp = &h->err;
   CK(cudaSetDevice(h->eng->dev));
-  void* d_n2d = nullptr;
-  const size_t bytes = sizeof(double) * 9 * (size_t)h->nl * h->nl * h->px * h->py;
-  int rc = dmalloc(errp, &d_n2d, bytes);
-  if (rc) return rc;
-  rc = tensor_real(h, static_cast<double*>(d_n2d));
-  if (!rc) {
-    cudaError_t ce = cudaMemcpy(n2d, d_n2d, bytes, cudaMemcpyDeviceToHost);
-    if (ce != cudaSuccess) rc = set_err(errp, MRM_ERR_CUDA, "download tensor: %s", cudaGetErrorString(ce));
-  }
-  dfree(d_n2d);
-  return rc;
+  TensorScratch w(h, false);
+  if (int rc = w.alloc(errp)) return rc;
+  if (int rc = tensor_real(h, w)) return rc;
+  CK(cudaStreamSynchronize(h->eng->st));
+  const cudaError_t ce = cudaMemcpy(n2d, w.at<double>(w.n2d), sizeof(double) * 9 * (size_t)h->nl * h->nl * h->px * h->py,
+                                    cudaMemcpyDeviceToHost);
+  if (ce != cudaSuccess) return set_err(errp, MRM_ERR_CUDA, "download tensor: %s", cudaGetErrorString(ce));
+  return MRM_OK;
 }
 
 int mrm_gpu_copy_tensor(mrm_gpu* dst, const mrm_gpu* src) {
