@@ -168,6 +168,10 @@ struct LayerDev {
   double gamma;
   int thermal;
   int n;
+  // 0: every record of pb (of xst) equals the first one, so a row kernel that
+  // reads them from global memory reads that one (one cached line in place of
+  // 16 B a grain); -1: a record per grain
+  int pb_mask, xs_mask;
 };
 
 // Device descriptor of one run (one medium realisation).

@@ -14,10 +14,17 @@
 // The spectrum buffer always holds H^(m) of the state it follows, so a step
 // starts from it without a separate demag pass.
 //
-// Latency layout: every per-grain global load (state, parameters, lattice
-// neighbours, columnar interlayer partner) is issued at the top of the row
-// kernel, before the inverse FFT, so its latency overlaps the shared-memory
-// passes; the column kernel batches its strided loads the same way.
+// What bounds the row kernel: on a batch, instruction issue (55 % of the slots)
+// and the latency of its grain loads; in a single run, whose 256 rows leave two
+// blocks to an SM, the chain copy -> inverse transform -> grains -> forward
+// transform of one row (about 1.5 + 2.3 + 2.5 + 2.6 us at 256 x 256).  Measured
+// per launch on 32 runs of 256 x 256 grains (predictor / corrector):
+// 126 / 126 us with two FFT buffers per sequence, the stage's scalars computed
+// by every thread, the spectrum post-processing one value at a time and a grain
+// record loaded per grain; 107 / 108 us with one buffer (rows transformed in
+// place), shared scalars, post-processing in pairs, uniform records read once,
+// waits without polling and two rows to a 128-thread block.  The two-layer
+// write's 1024-point rows, four blocks to an SM instead of two: 93 -> 56 us.
 #pragma once
 #include "common.cuh"
 #include "fft.cuh"
@@ -849,6 +856,8 @@ MRM_D double lds_r(const double* p) {
   asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(smem_u32(p)));
   return v;
 }
+MRM_D void sts_r(float* p, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(smem_u32(p)), "f"(v) : "memory"); }
+MRM_D void sts_r(double* p, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(smem_u32(p)), "d"(v) : "memory"); }
 
 // compile-time value selecting a generic lambda's instantiation
 template <int V>
@@ -894,24 +903,27 @@ MRM_HD RowStage row_stage_plan(int stage, int nx, int nrows, bool stencil, bool 
   return p;
 }
 
+// Register row transforms (FP32 runs, 16 <= M <= 1024 points); the choice
+// depends on M alone, so every row shape computes the same transform.
+MRM_HD constexpr bool rrow_len_ok(int lgM) { return lgM >= 4 && lgM <= 10; }
+template <typename R>
+MRM_HD constexpr bool row_reg(int lgM) { return sizeof(R) == sizeof(float) && rrow_len_ok(lgM); }
+
 // shared memory of the row kernel ahead of the grain staging area: twiddles
-// and the two FFT buffers sized for RPB rows
+// and the FFT buffers of RPB rows (one per sequence for the register
+// transforms, which work in place, else two)
 template <typename R>
 MRM_HD int row_fft_smem(int lgpx, int rpb) {
   const int M = 1 << (lgpx - 1);
-  return (row_tw_count(lgpx) + 2 * rpb * 3 * seq_stride(M)) * (int)sizeof(Cx<R>);
+  return (row_tw_count(lgpx) + (row_reg<R>(lgpx - 1) ? 1 : 2) * rpb * 3 * seq_stride(M)) * (int)sizeof(Cx<R>);
 }
 
-// Register row transforms of a block's sequences (FP32 runs, 16 <= M <= 1024
-// points): sequence s (= 3 row + component) at s * cs in each buffer, one group
-// of M/8 threads per sequence, group g taking sequences g, g + G, ...
-// (G = BLOCK / (M/8)).  The choice depends on M alone, so every row shape
-// computes the same transform.
-MRM_HD constexpr bool rrow_len_ok(int lgM) { return lgM >= 4 && lgM <= 10; }
-
+// The block's sequences: sequence s (= 3 row + component) at buf + s * cs, one
+// group of M/8 threads per sequence, group g taking sequences g, g + G, ...
+// (G = BLOCK / (M/8)).
 template <int LGM, int BLOCK>
-MRM_D void rrow_inverse_block(const Cx<float>* X, Cx<float>* xb, Cx<float>* out, int cs, int nseq, int nz,
-                              const Cx<float>* __restrict__ twpost, const Cx<float>* __restrict__ twpass) {
+MRM_D void rrow_inverse_block(Cx<float>* buf, int cs, int nseq, int nz, const Cx<float>* __restrict__ twpost,
+                              const Cx<float>* __restrict__ twpass) {
   constexpr int NT = 1 << (LGM - 3), G = BLOCK / NT;
   static_assert(G >= 1 && BLOCK % NT == 0, "whole groups per block");
   static_assert(NT <= 32 || G <= 4, "named barriers 1..4");
@@ -919,16 +931,12 @@ MRM_D void rrow_inverse_block(const Cx<float>* X, Cx<float>* xb, Cx<float>* out,
 #pragma unroll 1
   for (int s0 = 0; s0 < nseq; s0 += G) {
     const int s = s0 + g;
-    if (s < nseq) rrow_inverse<LGM>(X + s * cs, xb + s * cs, out + s * cs, t, g, nz, twpost, twpass);
+    if (s < nseq) rrow_inverse<LGM>(buf + s * cs, t, g, nz, twpost, twpass);
   }
 }
 
-// POST(s, t, nt, Y): the group's spectrum post-processing of sequence s from
-// its natural-order Y (the group is synchronised before and after the call's
-// reads through the next sequence's barriers; Y is not written again).
-template <int LGM, bool HALF, int BLOCK, class POST>
-MRM_D void rrow_forward_block(Cx<float>* in, Cx<float>* xb, int cs, int nseq, const Cx<float>* __restrict__ twpass,
-                              const POST& post) {
+template <int LGM, bool HALF, int BLOCK>
+MRM_D void rrow_forward_block(Cx<float>* buf, int cs, int nseq, const Cx<float>* __restrict__ twpass) {
   constexpr int NT = 1 << (LGM - 3), G = BLOCK / NT;
   static_assert(G >= 1 && BLOCK % NT == 0, "whole groups per block");
   static_assert(NT <= 32 || G <= 4, "named barriers 1..4");
@@ -936,39 +944,63 @@ MRM_D void rrow_forward_block(Cx<float>* in, Cx<float>* xb, int cs, int nseq, co
 #pragma unroll 1
   for (int s0 = 0; s0 < nseq; s0 += G) {
     const int s = s0 + g;
-    if (s < nseq) {
-      rrow_forward<LGM, HALF>(in + s * cs, xb + s * cs, in + s * cs, t, g, twpass);
-      post(s, t, NT, in + s * cs);
-    }
+    if (s < nseq) rrow_forward<LGM, HALF>(buf + s * cs, t, g, twpass);
   }
 }
 
 template <int BLOCK, int LGMAX>
-MRM_D void rrow_inverse_any(int lgM, const Cx<float>* X, Cx<float>* xb, Cx<float>* out, int cs, int nseq, int nz,
-                            const Cx<float>* twpost, const Cx<float>* twpass) {
+MRM_D void rrow_inverse_any(int lgM, Cx<float>* buf, int cs, int nseq, int nz, const Cx<float>* twpost,
+                            const Cx<float>* twpass) {
   switch (lgM) {
-    case 4: rrow_inverse_block<4, BLOCK>(X, xb, out, cs, nseq, nz, twpost, twpass); break;
-    case 5: rrow_inverse_block<5, BLOCK>(X, xb, out, cs, nseq, nz, twpost, twpass); break;
-    case 6: rrow_inverse_block<6, BLOCK>(X, xb, out, cs, nseq, nz, twpost, twpass); break;
-    case 7: if constexpr (LGMAX >= 8) rrow_inverse_block<7, BLOCK>(X, xb, out, cs, nseq, nz, twpost, twpass); break;
-    case 8: if constexpr (LGMAX >= 9) rrow_inverse_block<8, BLOCK>(X, xb, out, cs, nseq, nz, twpost, twpass); break;
-    case 9: if constexpr (LGMAX >= 10) rrow_inverse_block<9, BLOCK>(X, xb, out, cs, nseq, nz, twpost, twpass); break;
-    default: if constexpr (LGMAX >= 11) rrow_inverse_block<10, BLOCK>(X, xb, out, cs, nseq, nz, twpost, twpass); break;
+    case 4: rrow_inverse_block<4, BLOCK>(buf, cs, nseq, nz, twpost, twpass); break;
+    case 5: rrow_inverse_block<5, BLOCK>(buf, cs, nseq, nz, twpost, twpass); break;
+    case 6: rrow_inverse_block<6, BLOCK>(buf, cs, nseq, nz, twpost, twpass); break;
+    case 7: if constexpr (LGMAX >= 8) rrow_inverse_block<7, BLOCK>(buf, cs, nseq, nz, twpost, twpass); break;
+    case 8: if constexpr (LGMAX >= 9) rrow_inverse_block<8, BLOCK>(buf, cs, nseq, nz, twpost, twpass); break;
+    case 9: if constexpr (LGMAX >= 10) rrow_inverse_block<9, BLOCK>(buf, cs, nseq, nz, twpost, twpass); break;
+    default: if constexpr (LGMAX >= 11) rrow_inverse_block<10, BLOCK>(buf, cs, nseq, nz, twpost, twpass); break;
   }
 }
 
-template <int BLOCK, int LGMAX, bool HALF, class POST>
-MRM_D void rrow_forward_any(int lgM, Cx<float>* in, Cx<float>* xb, int cs, int nseq, const Cx<float>* twpass,
-                            const POST& post) {
+template <int BLOCK, int LGMAX, bool HALF>
+MRM_D void rrow_forward_any(int lgM, Cx<float>* buf, int cs, int nseq, const Cx<float>* twpass) {
   switch (lgM) {
-    case 4: rrow_forward_block<4, HALF, BLOCK>(in, xb, cs, nseq, twpass, post); break;
-    case 5: rrow_forward_block<5, HALF, BLOCK>(in, xb, cs, nseq, twpass, post); break;
-    case 6: rrow_forward_block<6, HALF, BLOCK>(in, xb, cs, nseq, twpass, post); break;
-    case 7: if constexpr (LGMAX >= 8) rrow_forward_block<7, HALF, BLOCK>(in, xb, cs, nseq, twpass, post); break;
-    case 8: if constexpr (LGMAX >= 9) rrow_forward_block<8, HALF, BLOCK>(in, xb, cs, nseq, twpass, post); break;
-    case 9: if constexpr (LGMAX >= 10) rrow_forward_block<9, HALF, BLOCK>(in, xb, cs, nseq, twpass, post); break;
-    default: if constexpr (LGMAX >= 11) rrow_forward_block<10, HALF, BLOCK>(in, xb, cs, nseq, twpass, post); break;
+    case 4: rrow_forward_block<4, HALF, BLOCK>(buf, cs, nseq, twpass); break;
+    case 5: rrow_forward_block<5, HALF, BLOCK>(buf, cs, nseq, twpass); break;
+    case 6: rrow_forward_block<6, HALF, BLOCK>(buf, cs, nseq, twpass); break;
+    case 7: if constexpr (LGMAX >= 8) rrow_forward_block<7, HALF, BLOCK>(buf, cs, nseq, twpass); break;
+    case 8: if constexpr (LGMAX >= 9) rrow_forward_block<8, HALF, BLOCK>(buf, cs, nseq, twpass); break;
+    case 9: if constexpr (LGMAX >= 10) rrow_forward_block<9, HALF, BLOCK>(buf, cs, nseq, twpass); break;
+    default: if constexpr (LGMAX >= 11) rrow_forward_block<10, HALF, BLOCK>(buf, cs, nseq, twpass); break;
   }
+}
+
+// The parts of a stage that every grain of the task shares: computed by one
+// thread (FP64 divisions and square roots, and the time functions, that each
+// thread used to take on its own between the inverse transform and the grain
+// loop).
+template <typename R>
+struct RowScalars {
+  double t_stage, sc, tps;  // the stage's time, the layer's time scale, the temperature profile's amplitude
+  R hax, hay, haz;          // uniform applied field (zero with a tabulated profile)
+  R tfac;                   // sqrt(T / dt)
+};
+template <typename R, int STAGE, int GEN>
+MRM_D void row_scalars(RowScalars<R>* o, const RunDev<R>& rd, const LayerDev<R>& L,
+                                                long long step, bool mid, bool ftab, bool thermal) {
+  const double t_now = rd.t_base + (double)(step - rd.step_base) * rd.dt;
+  const double t_st = (STAGE == kCorr) ? t_now + (mid ? 0.5 * rd.dt : rd.dt) : t_now;
+  const double sc = ramp(L, t_st);
+  // a layer's field is its uniform direction or its tabulated profile, scaled
+  double hd3[3] = {L.hdir[0], L.hdir[1], L.hdir[2]};
+  if (L.func == kFuncRot) rot_dir(L.fgamma, L.phase, t_st, hd3);
+  o->t_stage = t_st;
+  o->sc = sc;
+  o->tps = (GEN == 2 && L.tprof) ? L.tprof->dtemp * temp_scale(*L.tprof, t_st) : 0.0;
+  o->hax = ftab ? (R)0 : (R)(sc * hd3[0]);
+  o->hay = ftab ? (R)0 : (R)(sc * hd3[1]);
+  o->haz = ftab ? (R)0 : (R)(sc * hd3[2]);
+  o->tfac = thermal ? (R)sqrt(L.temperature / rd.dt) : (R)0;
 }
 
 // Row kernel: one task = up to RPB grid rows of one layer of one run (more for
@@ -992,6 +1024,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint64_t bars[3];
   __shared__ double sred[stats_slots<STAGE, STATS>()];
+  __shared__ RowScalars<R> scal;
   pdl_launch_dependents();
   const Task tk = tasks[blockIdx.x];
   const RunDev<R>& rd = runs[tk.x];
@@ -1019,7 +1052,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
   // longest may then have more than RPB rows per task (the host packs them
   // into the FFT buffers sized for the longest rows; not in level-2 batches)
   constexpr bool kRegRowType = sizeof(R) == sizeof(float);
-  const bool regrow = kRegRowType && rrow_len_ok(lgM);
+  const bool regrow = row_reg<R>(lgM);
+  const int nbuf = regrow ? 1 : 2;  // FFT buffers per sequence
   const int rcap = (GEN < 2 && regrow && !win) ? max(RPB, nrows) : RPB;
   const int nseq = nrows * 3;
   const int ngr = nrows * nx;
@@ -1031,23 +1065,23 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
 
   Cx<R>* tws = reinterpret_cast<Cx<R>*>(smem_raw);  // post twiddles | pass tables
   const int ntw = row_tw_count(lgpx);
-  if (nrows > rcap || (long long)(ntw + 2 * rcap * 3 * cs) * (long long)sizeof(Cx<R>) >
+  if (nrows > rcap || (long long)(ntw + nbuf * rcap * 3 * cs) * (long long)sizeof(Cx<R>) >
                           (long long)dynamic_smem_bytes()) {  // host bug: a task the buffers do not hold
     if (threadIdx.x == 0) atomicOr(err, kErrShape);
     return;
   }
   Cx<R>* bufA = tws + ntw;
-  Cx<R>* bufB = bufA + rcap * 3 * cs;
+  Cx<R>* bufB = regrow ? bufA : bufA + rcap * 3 * cs;  // holds the spectrum rows
+  unsigned char* fft_end = reinterpret_cast<unsigned char*>(bufA + nbuf * rcap * 3 * cs);
   // a layer under the moving write head gets its head field per grid column in
   // a table after the FFT buffers (the host reserves it), then the staging area
   // (its byte offset; 0: no head)
   // (a tabulated field profile gets its interpolation weights there instead)
   const bool ftab = GEN && STAGE != kInit && rd.L[tk.y].tab != nullptr;
   const int htab_off = GEN && (rd.L[tk.y].func == kFuncHead || ftab)
-                           ? (int)(reinterpret_cast<unsigned char*>(bufB + rcap * 3 * cs) - smem_raw)
+                           ? (int)(fft_end - smem_raw)
                            : 0;
-  unsigned char* stg = reinterpret_cast<unsigned char*>(bufB + rcap * 3 * cs) +
-                       (ftab ? field_table_bytes(rd.nx) : htab_off ? head_table_bytes<R>(rd.nx) : 0);
+  unsigned char* stg = fft_end + (ftab ? field_table_bytes(rd.nx) : htab_off ? head_table_bytes<R>(rd.nx) : 0);
   if (htab_off && (long long)(stg - smem_raw) > (long long)dynamic_smem_bytes()) {  // host bug: no room reserved
     if (threadIdx.x == 0) atomicOr(err, kErrShape);
     return;
@@ -1063,10 +1097,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
   const V4<R>* __restrict__ mfield = (STAGE == kCorr) ? L.mp : L.m;
   const V4<R>* __restrict__ mother_u = Lu ? ((STAGE == kCorr) ? Lu->mp : Lu->m) : nullptr;
   const V4<R>* __restrict__ mother_l = Ll ? ((STAGE == kCorr) ? Ll->mp : Ll->m) : nullptr;
-  const RowStage sp = row_stage_plan<R>(STAGE, nx, nrows, stencil, ucol, lcol, thermal);
   // staged when the plan fits both the launch's staging capacity and the
-  // shared memory actually allocated behind the FFT buffers
-  const bool staged = !win && sp.bytes <= stage_cap &&
+  // shared memory actually allocated behind the FFT buffers (the plan is only
+  // drawn up where the launch has a capacity)
+  const RowStage sp = stage_cap > 0 ? row_stage_plan<R>(STAGE, nx, nrows, stencil, ucol, lcol, thermal) : RowStage{};
+  const bool staged = !win && stage_cap > 0 && sp.bytes <= stage_cap &&
                       (long long)(stg - smem_raw) + sp.bytes <= (long long)dynamic_smem_bytes();
   const int base = win ? (wj0 + row0) * gnx + wi0 : row0 * nx;
   const int v4row = nx * (int)sizeof(V4<R>);
@@ -1115,10 +1150,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
     } else if (!win && v4row % 16 == 0) {
       // rows read at use: their parameter rows start for L2 now, and arrive
       // while the inverse row transforms run
-      bulk_prefetch_l2(L.pb + base, (uint32_t)(nrows * v4row));
+      if (GEN == 2 || L.pb_mask) bulk_prefetch_l2(L.pb + base, (uint32_t)(nrows * v4row));
       if (STAGE != kInit) {
         bulk_prefetch_l2(L.pa + base, (uint32_t)(nrows * v4row));
-        if (stencil) bulk_prefetch_l2(L.xst + base, (uint32_t)(nrows * v4row));
+        if (stencil && (GEN == 2 || L.xs_mask)) bulk_prefetch_l2(L.xst + base, (uint32_t)(nrows * v4row));
       }
     }
     mbar_arrive(&bars[0]);
@@ -1184,14 +1219,18 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
     return;
   }
 
+  // the stage's shared scalars, by the last warp: FP32 runs after the inverse
+  // transform, which leaves that warp idle unless the rows are long; FP64 ones
+  // while the rows' copies are on their way (every warp transforms there)
+  if (!kRegRowType && STAGE != kInit && threadIdx.x == BLOCK - 32)
+    row_scalars<R, STAGE, GEN>(&scal, rd, L, step, mid, ftab, thermal);
+
   // ---------------- inverse row transform: H^ rows -> H_demag ----------------
   Cx<R>* Z = bufA;  // after the inverse: z[n] = x[2n] + i x[2n+1] per sequence
   if (inverse && regrow) {
     if (leave_on_timeout(mbar_wait(&bars[0], 0) & mbar_wait(&bars[1], 0))) return;
     if constexpr (kRegRowType)
-      rrow_inverse_any<BLOCK, LGMAX>(lgM, bufB, bufA, bufB, cs, nseq, (nx + 1) >> 1, twpost, twpass);
-    __syncthreads();
-    Z = bufB;
+      rrow_inverse_any<BLOCK, LGMAX>(lgM, bufA, cs, nseq, (nx + 1) >> 1, twpost, twpass);
   } else if (inverse) {
     if (leave_on_timeout(mbar_wait(&bars[0], 0) & mbar_wait(&bars[1], 0))) return;
     const int tot = nseq * M;
@@ -1208,25 +1247,27 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
     __syncthreads();
     Z = block_fft_c<R, +1, NBMAX, BLOCK, LGMAX - 1>(bufA, bufB, lgM, nseq, twpass);
   }
-  Cx<R>* W = (Z == bufA) ? bufB : bufA;  // real outputs of this stage (forward input)
+  if (kRegRowType && STAGE != kInit && threadIdx.x == BLOCK - 32)
+    row_scalars<R, STAGE, GEN>(&scal, rd, L, step, mid, ftab, thermal);
+  // real outputs of this stage (forward input); with the register transforms
+  // each grain's moments replace its demag values
+  Cx<R>* W = (Z == bufA) ? bufB : bufA;
   const R* hdr = reinterpret_cast<const R*>(Z);
   R* outr = reinterpret_cast<R*>(W);
   const int rs = 2 * cs;  // real stride of one sequence
   if (leave_on_timeout(mbar_wait(&bars[0], 0) & mbar_wait(&bars[2], 0))) return;
 
   // ---------------- per-grain field + integrator stage ----------------
-  const double t_now = rd.t_base + (double)(step - rd.step_base) * rd.dt;
-  const double t_stage = (STAGE == kCorr) ? t_now + (mid ? 0.5 * rd.dt : rd.dt) : t_now;
-  const double sc = ramp(L, t_stage);
-  const double tps = (GEN == 2 && L.tprof) ? L.tprof->dtemp * temp_scale(*L.tprof, t_stage) : 0.0;
-  // a layer's field is its uniform direction or its tabulated profile, scaled
-  double hd3[3] = {L.hdir[0], L.hdir[1], L.hdir[2]};
-  if (L.func == kFuncRot) rot_dir(L.fgamma, L.phase, t_stage, hd3);
-  const R hax = ftab ? (R)0 : (R)(sc * hd3[0]), hay = ftab ? (R)0 : (R)(sc * hd3[1]),
-          haz = ftab ? (R)0 : (R)(sc * hd3[2]);
+  // (kInit only needs the time, for temperature scaling)
+  const double t_now = (GEN == 2 || STAGE == kInit) ? rd.t_base + (double)(step - rd.step_base) * rd.dt : 0.0;
+  const double t_stage = STAGE == kInit ? t_now : scal.t_stage;
+  const double sc = STAGE == kInit ? 0.0 : scal.sc;
+  const double tps = STAGE == kInit ? 0.0 : scal.tps;
+  const R hax = STAGE == kInit ? (R)0 : scal.hax, hay = STAGE == kInit ? (R)0 : scal.hay,
+          haz = STAGE == kInit ? (R)0 : scal.haz;
   const R dt = (R)rd.dt;
   const R gamma = (R)L.gamma;
-  const R tfac = thermal ? (R)sqrt(L.temperature / rd.dt) : (R)0;  // sqrt(T/dt)
+  const R tfac = STAGE == kInit ? (R)0 : scal.tfac;  // sqrt(T/dt)
   // (a demag-only evaluation leaves L.hf alone: it holds the last stepping
   // stage's field, which a retried adaptive step reads)
   const bool store_field = (flags & kFlagStoreField) || (STAGE == kEval && !(flags & kFlagDemagOnly));
@@ -1294,9 +1335,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
   constexpr int MODE = decltype(mode_c)::value;
   const bool ST = MODE == 2 ? staged : MODE == 1;
   auto srow = [&](int off) { return reinterpret_cast<const V4<R>*>(stg + off); };
-  const V4<R>* PB = ST ? srow(sp.pb) : L.pb + base;
+  // (uniform records: LayerDev; the level-2 kernels have no register to spare for them)
+  const int pbm = ST || GEN == 2 ? -1 : L.pb_mask, xsm = ST || GEN == 2 ? -1 : L.xs_mask;
+  const V4<R>* PB = ST ? srow(sp.pb) : pbm ? L.pb + base : L.pb;
   const V4<R>* PA = ST ? srow(sp.pa) : L.pa + base;
-  const V4<R>* XS = ST ? srow(sp.xst) : L.xst + base;
+  const V4<R>* XS = ST ? srow(sp.xst) : xsm ? L.xst + base : L.xst;
   const R* UC = (ST && sp.ucol >= 0) ? reinterpret_cast<const R*>(stg + sp.ucol) : (ucol ? L.ucol + base : nullptr);
   const R* LC = (ST && sp.lcol >= 0) ? reinterpret_cast<const R*>(stg + sp.lcol) : (lcol ? L.lcol + base : nullptr);
   const V4<R>* MF = ST ? srow(sp.mf) + sp.halo * nx : mfield + base;
@@ -1328,16 +1371,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
     if constexpr (MODE == 1) return lds_v4(p + i);
     else return p[i];
   };
-  auto at1 = [&](const R* p, int i) -> R {
-    if constexpr (MODE == 1) return lds_r(p + i);
-    else return p[i];
-  };
   for (int idx = threadIdx.x; idx < ngr; idx += BLOCK) {
     const int rr = pow2x ? (idx >> lgnx) : idx / nx;
     const int i = idx - rr * nx;
     const int q = idx;                // index within the task's rows
     const int n = base + idx;         // grain index within the layer
-    V4<R> pb = at4(PB, q);
+    V4<R> pb = at4(PB, q & pbm);
     // (temperature scaling, level 2: the grain's grid cell)
     const int gi = wi0 + i, gj = wj0 + row0 + rr;
     if (STAGE == kInit) {
@@ -1345,9 +1384,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
       R ms0 = pb.x;  // Ms * ms_scale
       if constexpr (GEN == 2)
         if (L.tsc) ms0 = (R)((double)pb.x * tsc_ms(*L.tsc, n, layer_temp(L, t_stage, gi, gj), (double)mf.w));
-      outr[(rr * 3 + 0) * rs + i] = ms0 * mf.x;
-      outr[(rr * 3 + 1) * rs + i] = ms0 * mf.y;
-      outr[(rr * 3 + 2) * rs + i] = ms0 * mf.z;
+      sts_r(outr + (rr * 3 + 0) * rs + i, ms0 * mf.x);
+      sts_r(outr + (rr * 3 + 1) * rs + i, ms0 * mf.y);
+      sts_r(outr + (rr * 3 + 2) * rs + i, ms0 * mf.z);
       continue;
     }
     const V4<R> mf = at4(MF, q);
@@ -1381,9 +1420,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
       hdy = g.y;
       hdz = g.z;
     } else if (use_hdr) {
-      hdx = at1(hdr, (rr * 3 + 0) * rs + i);
-      hdy = at1(hdr, (rr * 3 + 1) * rs + i);
-      hdz = at1(hdr, (rr * 3 + 2) * rs + i);
+      hdx = lds_r(hdr + (rr * 3 + 0) * rs + i);
+      hdy = lds_r(hdr + (rr * 3 + 1) * rs + i);
+      hdz = lds_r(hdr + (rr * 3 + 2) * rs + i);
     }
     // applied field of this grain: the uniform part (plus the write head's in
     // the evaluation stage; the stepping stages carry it in hdx, hdz)
@@ -1444,7 +1483,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
     }
     R ex = 0, ey = 0, ez = 0;
     if (stencil) {
-      V4<R> c = at4(XS, q);
+      V4<R> c = at4(XS, q & xsm);
       const V4<R>* rowc = mf_row(rr);
       // (in a window the neighbours are the full grid's: row pointers at the
       // full rows' starts, the grid column wi0 + i)
@@ -1691,12 +1730,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
     if constexpr (GEN == 2) {
       if (L.tsc) {
         const double t_src = (STAGE == kPred && mid) ? t_now + 0.5 * rd.dt : t_now + rd.dt;
-        msrc = (R)((double)at4(PB, q).x * tsc_ms(*L.tsc, n, layer_temp(L, t_src, gi, gj), (double)mn.w));
+        msrc = (R)((double)at4(PB, q & pbm).x * tsc_ms(*L.tsc, n, layer_temp(L, t_src, gi, gj), (double)mn.w));
       }
     }
-    outr[(rr * 3 + 0) * rs + i] = msrc * mn.x;
-    outr[(rr * 3 + 1) * rs + i] = msrc * mn.y;
-    outr[(rr * 3 + 2) * rs + i] = msrc * mn.z;
+    sts_r(outr + (rr * 3 + 0) * rs + i, msrc * mn.x);
+    sts_r(outr + (rr * 3 + 1) * rs + i, msrc * mn.y);
+    sts_r(outr + (rr * 3 + 2) * rs + i, msrc * mn.z);
 
     if constexpr (stats) {
       const V4<double> pv = L.pv[n];  // {vol, ms_scale, ms, 1}; (0, .., 0) on the extra cells of a grain
@@ -1754,35 +1793,44 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
       for (int i = nx + threadIdx.x; i < zlim; i += BLOCK) outr[s * rs + i] = (R)0;
   }
   __syncthreads();
-  Cx<R>* scratch = (W == bufA) ? bufB : bufA;
   const int nys = rd.nys, lgct = rd.lgct, T = 1 << lgct, ntile = (ph + T - 1) >> lgct;
   if constexpr (kRegRowType) {
     if (regrow) {
-      // X[k] = e - i w^k o (w = e^{-2 pi i / px}) for the group's sequence:
-      // thread t takes k = t + j M/8 (and k = M), stored in column tiles of
-      // T = 2^lgct columns, each tile row by row
-      auto post = [&](int s, int t, int nt, const Cx<R>* Ys) {
+      if (half_in) rrow_forward_any<BLOCK, LGMAX, true>(lgM, W, cs, nseq, twpass);
+      else rrow_forward_any<BLOCK, LGMAX, false>(lgM, W, cs, nseq, twpass);
+      __syncthreads();
+      // X[k] = e - i w^k o (w = e^{-2 pi i / px}) and X[M-k] = conj(e) - i
+      // conj(w^k o) from the pair Y[k], Y[M-k], by all threads of the block
+      // (X[0] and X[M] from Y[0]; the thread of k = 0 takes X[M/2] as well),
+      // stored in column tiles of T = 2^lgct columns, each tile row by row
+      const int lgp = lgM - 1, npair = nseq << lgp;
+      for (int idx = threadIdx.x; idx < npair; idx += BLOCK) {
+        const int s = idx >> lgp, k = idx & ((1 << lgp) - 1);
         const int row = s / 3, comp = s - 3 * row;
+        const Cx<R>* Ys = W + s * cs;
         Cx<R>* dst = rd.specx + (size_t)(l * 3 + comp) * ntile * nys * T;
-#pragma unroll 1
-        for (int k = t; k <= M; k += nt) {
-          const Cx<R> yk = Ys[k & (M - 1)];
-          const Cx<R> ymk = cconj(Ys[(M - k) & (M - 1)]);
-          const Cx<R> e = cscale(cadd(yk, ymk), (R)0.5);
-          const Cx<R> o = cscale(csub(yk, ymk), (R)0.5);
-          const Cx<R> wo = cmul(twpost[k], o);
-          const long long at = (((long long)(k >> lgct) * nys + row0 + row) << lgct) + (k & (T - 1));
+        auto put = [&](int kk, Cx<R> x) {
+          const long long at = (((long long)(kk >> lgct) * nys + row0 + row) << lgct) + (kk & (T - 1));
           if (!MRM_CHECK((long long)(l * 3 + comp) * ntile * nys * T + at < (long long)rd.nl * 3 * ntile * nys * T,
-                         310, k))
-            continue;
-          dst[at] = csub(e, cmul_i(wo, (R)1));
+                         310, kk))
+            return;
+          dst[at] = x;
+        };
+        const Cx<R> yk = Ys[k], ymk = cconj(Ys[(M - k) & (M - 1)]);
+        const Cx<R> e = cscale(cadd(yk, ymk), (R)0.5);
+        const Cx<R> o = cscale(csub(yk, ymk), (R)0.5);
+        const Cx<R> wo = cmul(twpost[k], o);
+        put(k, Cx<R>{e.x + wo.y, e.y - wo.x});
+        put(M - k, Cx<R>{e.x - wo.y, -e.y - wo.x});
+        if (k == 0) {  // Y[M/2] pairs with itself: X[M/2] = conj(Y[M/2])
+          const Cx<R> h = Ys[M >> 1];
+          put(M >> 1, cconj(h));
         }
-      };
-      if (half_in) rrow_forward_any<BLOCK, LGMAX, true>(lgM, W, scratch, cs, nseq, twpass, post);
-      else rrow_forward_any<BLOCK, LGMAX, false>(lgM, W, scratch, cs, nseq, twpass, post);
+      }
       return;
     }
   }
+  Cx<R>* scratch = (W == bufA) ? bufB : bufA;
   Cx<R>* Y = block_fft_c<R, -1, NBMAX, BLOCK, LGMAX - 1>(W, scratch, lgM, nseq, twpass);
   // X[k] = e - i w^k o (w = e^{-2 pi i / px}), stored in column tiles of T =
   // 2^lgct columns (one column task), each tile row by row: consecutive threads

@@ -51,6 +51,7 @@ struct LayerBufs {
   int *lidx = nullptr, *lnbr = nullptr;
   void* lcoef = nullptr;
   void* xst = nullptr;   // V4<R> lattice exchange coefficients (null: CSR form)
+  bool pb_uniform = false, xst_uniform = false;  // every record equal, bit for bit
   void* cax = nullptr;   // V4<R> x 3 per grain: cubic crystal axes (null: uniaxial)
   void* ucol = nullptr;  // R columnar interlayer coefficients (null: CSR form)
   void* lcol = nullptr;
@@ -432,7 +433,7 @@ constexpr int kSlots = kRowSlots;
 constexpr int kSlotStage[kSlots] = {kInit, kPred, kCorr, kCorr, kEval, kPred};
 // static shared memory of a row stage (mbarriers, reduction scratch) with margin
 size_t row_static_bytes(int slot) {
-  return ((slot == 3 || slot == 5) ? 32 * kNPart * sizeof(double) : sizeof(double)) + 64;
+  return ((slot == 3 || slot == 5) ? 32 * kNPart * sizeof(double) : sizeof(double)) + 128;
 }
 constexpr size_t kSmemPerSM = 228 * 1024;
 constexpr size_t kSmemReserved = 1024;  // per block
@@ -626,6 +627,8 @@ RunDev<R> make_desc(const mrm_gpu* r) {
     o.lnbr = b.lnbr;
     o.lcoef = static_cast<const R*>(b.lcoef);
     o.xst = static_cast<const V4<R>*>(b.xst);
+    o.pb_mask = b.pb_uniform ? 0 : -1;
+    o.xs_mask = b.xst_uniform ? 0 : -1;
     o.cax = static_cast<const V4<R>*>(b.cax);
     o.cgrain = b.cgrain;
     o.gci = b.gci;
@@ -709,7 +712,7 @@ int plan_smem(Engine* e) {
   std::string* errp = &e->err;
   const RowVariant rv = row_variant<R>(e->rowv);
   size_t fft = 16;
-  int need[kSlots] = {0, 0, 0, 0, 0, 0};
+  int need[kSlots] = {0, 0, 0, 0, 0, 0}, least[kSlots] = {0, 0, 0, 0, 0, 0};
   size_t scol = 16;
   int tw_cap = 0, stage_bytes = 0;
   const RowPackCap pack = row_pack_cap<R>(e, rv.rpb);
@@ -718,7 +721,11 @@ int plan_smem(Engine* e) {
       return set_err(errp, MRM_ERR_UNSUPPORTED, "row shape %d does not cover %d-column FFT grids", e->rowv, r->px);
     const int rows = rows_per_task<R>(r, rv.rpb, pack);
     fft = std::max(fft, row_fixed_smem<R>(r, rv.rpb));
-    for (int q = 0; q < kSlots; ++q) need[q] = std::max(need[q], run_stage_bytes<R>(r, kSlotStage[q], rows));
+    for (int q = 0; q < kSlots; ++q) {
+      const int bytes = run_stage_bytes<R>(r, kSlotStage[q], rows);
+      need[q] = std::max(need[q], bytes);
+      least[q] = least[q] ? std::min(least[q], bytes) : bytes;
+    }
     if (r->demag && r->tensor_ready) {
       if (creg_run(r)) {
         tw_cap = std::max(tw_cap, col_tw_count(r->lgpy));
@@ -731,7 +738,9 @@ int plan_smem(Engine* e) {
                                 (long long)row_static_bytes(q) - (long long)fft;
     const long long hard = (long long)kMaxSmem - (long long)row_static_bytes(q) - (long long)fft;
     if (hard < 0) return set_err(errp, MRM_ERR_UNSUPPORTED, "row shape %d exceeds shared memory", e->rowv);
-    const long long cap = std::min<long long>(need[q], std::max(0LL, std::min(per_block, hard)));
+    // (a capacity that no run's rows fit is none)
+    long long cap = std::min<long long>(need[q], std::max(0LL, std::min(per_block, hard)));
+    if (cap < least[q]) cap = 0;
     e->stage_cap[q] = (int)(cap & ~15LL);
     e->smem_row[q] = fft + (size_t)e->stage_cap[q];
   }
@@ -1556,6 +1565,14 @@ int upload_csr(mrm_gpu* r, int n, const int32_t* index, const int32_t* grain, co
   return MRM_OK;
 }
 
+// whether every four-value record equals the first, bit for bit
+template <typename R>
+bool uniform_records(const std::vector<R>& v) {
+  for (size_t i = 4; i < v.size(); i += 4)
+    if (std::memcmp(&v[i], &v[0], 4 * sizeof(R)) != 0) return false;
+  return true;
+}
+
 // host copies of ms_scale per layer (neighbour scaling of exchange coefficients)
 struct HostLayerCache {
   std::vector<double> ms_scale, ms, hk_scale, vol, alpha_scale;  // per grain
@@ -1645,6 +1662,7 @@ int upload_layer_t(mrm_gpu* r, int l, int n, const double* ms, const double* vol
   LayerBufs& b = r->L[l];
   CK(h2d(b.pa, pa.data(), sizeof(R) * 4 * nc));
   CK(h2d(b.pb, pb.data(), sizeof(R) * 4 * nc));
+  b.pb_uniform = uniform_records(pb);
   CK(h2d(b.pv, pv.data(), sizeof(double) * 4 * nc));
   auto& hc = host_cache()[r];
   hc.resize(MRM_MAX_LAYERS);
@@ -1721,6 +1739,7 @@ int upload_layer_t(mrm_gpu* r, int l, int n, const double* ms, const double* vol
       int rc2 = dmalloc(errp, &b.xst, sizeof(R) * 4 * (size_t)n);
       if (rc2) return rc2;
       CK(h2d(b.xst, st.data(), sizeof(R) * 4 * (size_t)n));
+      b.xst_uniform = uniform_records(st);
     }
   } else {
     dfree(b.xidx); dfree(b.xnbr); dfree(b.xcoef);

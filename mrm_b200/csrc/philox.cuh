@@ -38,8 +38,9 @@ MRM_D void philox4x32_10(unsigned int c[4], unsigned int k0, unsigned int k1) {
   const unsigned int W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
 #pragma unroll
   for (int r = 0; r < 10; ++r) {
-    const unsigned int hi0 = __umulhi(M0, c[0]), lo0 = M0 * c[0];
-    const unsigned int hi1 = __umulhi(M1, c[2]), lo1 = M1 * c[2];
+    const unsigned long long p0 = (unsigned long long)M0 * c[0], p1 = (unsigned long long)M1 * c[2];
+    const unsigned int hi0 = (unsigned int)(p0 >> 32), lo0 = (unsigned int)p0;
+    const unsigned int hi1 = (unsigned int)(p1 >> 32), lo1 = (unsigned int)p1;
     const unsigned int n0 = hi1 ^ c[1] ^ k0;
     const unsigned int n2 = hi0 ^ c[3] ^ k1;
     c[0] = n0;

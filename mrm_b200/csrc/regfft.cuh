@@ -171,7 +171,7 @@ MRM_D void reg_sync(int c) {
 // One stage on a single sequence in its exchange buffer b (in place at the
 // thread's positions of the stage).
 template <int LGN, int STAGE, bool INV>
-MRM_D void reg_stage1(Cx<float>* __restrict__ b, int t, const Cx<float>* __restrict__ tw) {
+MRM_D void reg_stage1(Cx<float>* b, int t, const Cx<float>* __restrict__ tw) {
   using P = RegPlan<LGN>;
   constexpr int B = P::dbit(STAGE);
   Cx<float> w[8];
@@ -194,15 +194,19 @@ MRM_D void reg_stage1(Cx<float>* __restrict__ b, int t, const Cx<float>* __restr
 // for Y = FFT_M(z), w = e^{-2 pi i / 2M}; the inverse forms Z[k] = e + i w^-k o,
 // e = X[k] + conj X[M-k], o = X[k] - conj X[M-k], and z = IFFT_M(Z).
 
-// Inverse: X (M + 1 spectrum values, natural order) -> z[n] for n < nz into
-// out; xb: the sequence's exchange buffer (M elements).  Thread t gathers the
-// pre-processed spectrum at its first stage's positions, the digit-reversed
-// frequencies ft + k M/8 (ft = ip_freq(8t)), so no reordering pass is needed.
-// out may be X itself: every gather is behind at least one barrier of the
-// group (LGM >= 4: two or more stages).
+// Both transforms work in place in the sequence's one buffer: every stage's
+// loads are behind a barrier of the group before another thread's positions
+// are overwritten.  (A second buffer saved one barrier per transform and cost
+// half the resident blocks of the long rows: two 1024-point rows' blocks per
+// SM instead of four.)
+
+// Inverse: b holds X (M + 1 spectrum values, natural order) -> z[n] for n < nz.
+// Thread t gathers the pre-processed spectrum at its first stage's positions,
+// the digit-reversed frequencies ft + k M/8 (ft = ip_freq(8t)), so no
+// reordering pass is needed.
 template <int LGM>
-MRM_D void rrow_inverse(const Cx<float>* X, Cx<float>* __restrict__ xb, Cx<float>* out, int t, int g, int nz,
-                        const Cx<float>* __restrict__ twpost, const Cx<float>* __restrict__ twpass) {
+MRM_D void rrow_inverse(Cx<float>* b, int t, int g, int nz, const Cx<float>* __restrict__ twpost,
+                        const Cx<float>* __restrict__ twpass) {
   using P = RegPlan<LGM>;
   constexpr int M = P::N, NT = P::NT, S = P::S;
   static_assert(S >= 2, "a barrier between the gather and the output");
@@ -211,13 +215,13 @@ MRM_D void rrow_inverse(const Cx<float>* X, Cx<float>* __restrict__ xb, Cx<float
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const int f = ft + k * NT;
-    Cx<float> a = X[f], b = X[M - f];
+    Cx<float> x = b[f], y = b[M - f];
     if (f == 0) {  // self-conjugate bins: imaginary parts ignored (c2r)
-      a.y = 0.f;
-      b.y = 0.f;
+      x.y = 0.f;
+      y.y = 0.f;
     }
-    const Cx<float> e = cadd(a, cconj(b));
-    const Cx<float> o = csub(a, cconj(b));
+    const Cx<float> e = cadd(x, cconj(y));
+    const Cx<float> o = csub(x, cconj(y));
     const Cx<float> w = cconj(twpost[f]);  // e^{+2 pi i f / 2M}
     v[k] = cadd(e, cmul_i(cmul(o, w), 1.f));
   }
@@ -225,17 +229,18 @@ MRM_D void rrow_inverse(const Cx<float>* X, Cx<float>* __restrict__ xb, Cx<float
     Cx<float> w[8];
     reg_twiddles<LGM, S - 1>(w, t, twpass);
     reg_inv<LGM, S - 1>(v, w);
+    reg_sync<NT>(g);
     const int a = xswz(t << 3);  // stage S-1 positions 8t + k
 #pragma unroll
-    for (int k = 0; k < 8; ++k) xb[a ^ k] = v[k];
+    for (int k = 0; k < 8; ++k) b[a ^ k] = v[k];
   }
   reg_sync<NT>(g);
   if constexpr (S >= 4) {
-    reg_stage1<LGM, 2, true>(xb, t, twpass);
+    reg_stage1<LGM, 2, true>(b, t, twpass);
     reg_sync<NT>(g);
   }
   if constexpr (S >= 3) {
-    reg_stage1<LGM, 1, true>(xb, t, twpass);
+    reg_stage1<LGM, 1, true>(b, t, twpass);
     reg_sync<NT>(g);
   }
   Cx<float> w[8];
@@ -243,56 +248,56 @@ MRM_D void rrow_inverse(const Cx<float>* X, Cx<float>* __restrict__ xb, Cx<float
   constexpr int B0 = P::dbit(0);
   const int a = xswz(reg_base<B0>(t));
 #pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = xb[a ^ xswz(k << B0)];
+  for (int k = 0; k < 8; ++k) v[k] = b[a ^ xswz(k << B0)];
   reg_inv<LGM, 0>(v, w);
+  reg_sync<NT>(g);
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const int n = t + k * NT;  // stage 0 positions: natural order
-    if (n < nz) out[n] = v[k];
+    if (n < nz) b[n] = v[k];
   }
 }
 
-// Forward: z (natural order, n < M; HALF: zero for n >= M/2 and not read) ->
-// Y = FFT_M(z) in natural order into nat, which may be the input itself (every
-// load is behind at least one barrier of the group); xb: the exchange buffer.
-// The group's threads are synchronised on return.
+// Forward: z in b (natural order, n < M; HALF: zero for n >= M/2 and not read)
+// -> Y = FFT_M(z) in natural order.  (The caller synchronises the block before
+// Y is read.)
 template <int LGM, bool HALF>
-MRM_D void rrow_forward(const Cx<float>* in, Cx<float>* __restrict__ xb, Cx<float>* nat, int t, int g,
-                        const Cx<float>* __restrict__ twpass) {
+MRM_D void rrow_forward(Cx<float>* b, int t, int g, const Cx<float>* __restrict__ twpass) {
   using P = RegPlan<LGM>;
   constexpr int NT = P::NT, S = P::S, KIN = HALF ? 4 : 8;
   static_assert(S >= 2, "a barrier between the loads and the output");
   Cx<float> v[8];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = k < KIN ? in[t + k * NT] : Cx<float>{0.f, 0.f};
+  for (int k = 0; k < 8; ++k) v[k] = k < KIN ? b[t + k * NT] : Cx<float>{0.f, 0.f};
   {
     Cx<float> w[8];
     reg_twiddles<LGM, 0>(w, t, twpass);
     reg_fwd<LGM, 0, HALF>(v, w);
+    reg_sync<NT>(g);
     constexpr int B0 = P::dbit(0);
     const int a = xswz(reg_base<B0>(t));
 #pragma unroll
-    for (int k = 0; k < 8; ++k) xb[a ^ xswz(k << B0)] = v[k];
+    for (int k = 0; k < 8; ++k) b[a ^ xswz(k << B0)] = v[k];
   }
   reg_sync<NT>(g);
   if constexpr (S >= 3) {
-    reg_stage1<LGM, 1, false>(xb, t, twpass);
+    reg_stage1<LGM, 1, false>(b, t, twpass);
     reg_sync<NT>(g);
   }
   if constexpr (S >= 4) {
-    reg_stage1<LGM, 2, false>(xb, t, twpass);
+    reg_stage1<LGM, 2, false>(b, t, twpass);
     reg_sync<NT>(g);
   }
   Cx<float> w[8];
   reg_twiddles<LGM, S - 1>(w, t, twpass);
   const int a = xswz(t << 3);
 #pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = xb[a ^ k];
+  for (int k = 0; k < 8; ++k) v[k] = b[a ^ k];
   reg_fwd<LGM, S - 1, false>(v, w);
   const int ft = ip_freq(8 * t, LGM);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) nat[ft + k * NT] = v[k];
   reg_sync<NT>(g);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) b[ft + k * NT] = v[k];
 }
 
 }  // namespace mrm

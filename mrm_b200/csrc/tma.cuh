@@ -58,14 +58,18 @@ MRM_D void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
                : "memory");
 }
 
+// (the thread may be suspended for up to kWaitHintNs before a failed poll
+// returns: without the hint a block waiting for a copy spent a twentieth of
+// the row kernel's issue slots on polls)
+constexpr uint32_t kWaitHintNs = 20000;
 MRM_D bool mbar_try_wait(uint64_t* bar, uint32_t phase) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(phase)
+      : "r"(smem_u32(bar)), "r"(phase), "r"(kWaitHintNs)
       : "memory");
   return ok != 0;
 }
