@@ -1,5 +1,6 @@
 // common.cuh -- device types shared by the grain-dynamics kernels (sm_100a).
 #pragma once
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -176,7 +177,7 @@ struct LayerDev {
 
 // Device descriptor of one run (one medium realisation).
 template <typename R>
-struct RunDev {
+struct alignas(16) RunDev {
   int nx, ny, nl;
   int px, py, lgpx, lgpy;  // FFT grid (px = 2^lgpx)
   int demag;
@@ -206,6 +207,9 @@ struct RunDev {
                            // FP64 full [px/2+1][nl*nl][9][py] complex
   LayerDev<R> L[kMaxLayers];
 };
+
+// the part of a run's descriptor ahead of its layers, in whole 16-byte units
+constexpr int kRunHdrBytes = (int)((offsetof(RunDev<float>, L) + 15) / 16 * 16);
 
 constexpr int kFuncHead = 6;
 constexpr int kFuncRot = 7;  // the ROT time function: an in-plane field rotating at rate gamma

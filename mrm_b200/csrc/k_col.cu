@@ -177,32 +177,38 @@ template <>
 cudaError_t col_occupancy<double>(int v, size_t smem, int* blocks) { return col_occ_any<double>(v, smem, blocks); }
 
 // ---------------- register column kernel shapes (k_creg_*.cu) ----------------
-static const ColOps* creg_ops_of(int v) {
+static const CregOps* creg_ops_of(int v, int nl) {
+  if (nl < 1 || nl > 2) return nullptr;
   switch (v) {
     case 0: return &creg_ops<0>();
     case 1: return &creg_ops<1>();
     case 2: return &creg_ops<2>();
+    case 3: return &creg_ops<3>();
     default: return nullptr;
   }
 }
-cudaError_t launch_creg(int v, const ColLaunch& a, int istep, int flags) {
-  const ColOps* o = creg_ops_of(v);
-  return o ? o->launch(a, istep, flags) : cudaErrorInvalidValue;
+cudaError_t launch_creg(int v, int nl, const ColLaunch& a, int istep, int flags) {
+  const CregOps* o = creg_ops_of(v, nl);
+  return o ? o->launch[nl - 1](a, istep, flags) : cudaErrorInvalidValue;
 }
-cudaError_t creg_allow_smem(int v, size_t smem) {
-  const ColOps* o = creg_ops_of(v);
-  return o ? allow_smem(o->fn, smem) : cudaErrorInvalidValue;
+cudaError_t creg_allow_smem(int v, int nl, size_t smem) {
+  const CregOps* o = creg_ops_of(v, nl);
+  return o ? allow_smem(o->fn[nl - 1], smem) : cudaErrorInvalidValue;
 }
-cudaError_t creg_occupancy(int v, size_t smem, int* blocks) {
-  const ColOps* o = creg_ops_of(v);
-  return o ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, o->fn, kCreg[v].block, smem)
+cudaError_t creg_occupancy(int v, int nl, size_t smem, int* blocks) {
+  const CregOps* o = creg_ops_of(v, nl);
+  return o ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, o->fn[nl - 1], creg_block(v, nl), smem)
            : cudaErrorInvalidValue;
 }
 cudaError_t creg_load(int v) {
-  const ColOps* o = creg_ops_of(v);
-  if (!o) return cudaErrorInvalidValue;
   cudaFuncAttributes fa;
-  return cudaFuncGetAttributes(&fa, o->fn);
+  for (int nl = 1; nl <= 2; ++nl) {
+    const CregOps* o = creg_ops_of(v, nl);
+    if (!o) return cudaErrorInvalidValue;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, o->fn[nl - 1]);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 template <typename R>

@@ -40,13 +40,25 @@ template <typename R>
 constexpr ColVariant col_variant(int v) { return sizeof(R) == sizeof(float) ? kColF32[v] : kColF64[v]; }
 
 // Register column kernel shapes (colreg.cuh: FP32 runs of one layer with
-// 256..1024-point columns); the column shape index selects one of these for
-// those runs and one of kColF32 for the others.
+// 64..1024-point columns or of two with 512 or 1024); the column shape index selects one of these
+// for those runs and one of kColF32 for the others.  For runs of nl layers: the
+// threads of a component group, which holds columns of at most 8 times as many
+// points (shape 0 takes every length), the resident blocks, and whether one
+// group takes the components in turn (else 3 nl groups, one each).
 struct CregVariant {
-  int block, minb;
+  int group[2], minb[2];
+  bool serial[2];
 };
-constexpr int kCregVariants = 3;
-constexpr CregVariant kCreg[kCregVariants] = {{128, 4}, {256, 2}, {128, 5}};
+constexpr int kCregVariants = 3, kCregShapes = 4;
+constexpr CregVariant kCreg[kCregShapes] = {{{128, 128}, {2, 1}, {false, false}},
+                                            {{64, 64}, {2, 2}, {false, false}},
+                                            {{128, 64}, {3, 2}, {true, false}},
+                                            {{32, 64}, {2, 2}, {false, false}}};
+// column shape 1 where no column is longer than its groups hold: half the
+// columns to a block spread a single run's few tasks over twice the blocks
+// (200 x 75 grains: 36.0 -> 34.6 us per step)
+constexpr int kCregShort = 3;
+constexpr int creg_block(int v, int nl) { return kCreg[v].group[nl - 1] * (kCreg[v].serial[nl - 1] ? 1 : 3 * nl); }
 
 struct RowLaunch;
 // entry points of one compiled row shape (defined in its own translation unit)
@@ -106,9 +118,14 @@ struct ColOps {
 };
 template <typename R, int V>
 const ColOps& col_ops();
-// entry points of one register column kernel shape (k_creg_*.cu)
+// entry points of one register column kernel shape (k_creg_*.cu), for runs of
+// one and of two layers
+struct CregOps {
+  cudaError_t (*launch[2])(const ColLaunch& a, int istep, int flags);
+  const void* fn[2];
+};
 template <int V>
-const ColOps& creg_ops();
+const CregOps& creg_ops();
 
 // stage: kInit, kPred, kCorr, kEval; stats selects the corrector with reductions
 template <typename R>
@@ -140,10 +157,10 @@ template <typename R>
 cudaError_t col_occupancy(int variant, size_t smem, int* blocks_per_sm);
 template <typename R>
 cudaError_t col_load(int variant);
-// the register column kernel (FP32)
-cudaError_t launch_creg(int variant, const ColLaunch& a, int istep, int flags);
-cudaError_t creg_allow_smem(int variant, size_t smem);
-cudaError_t creg_occupancy(int variant, size_t smem, int* blocks_per_sm);
+// the register column kernel (FP32) for runs of nl = 1 or 2 layers
+cudaError_t launch_creg(int variant, int nl, const ColLaunch& a, int istep, int flags);
+cudaError_t creg_allow_smem(int variant, int nl, size_t smem);
+cudaError_t creg_occupancy(int variant, int nl, size_t smem, int* blocks_per_sm);
 cudaError_t creg_load(int variant);
 
 // launches with or without programmatic stream serialization

@@ -116,6 +116,7 @@ struct mrm_gpu {
   bool tensor_ready = false;
   bool demag = true;
   double tensor_resid = 0.0, tensor_kept = 0.0;
+  bool tens_sym = true;  // each layer pair's tensor spectrum is symmetric (see creg_run)
   double dt = 1e-13, t_base = 0.0;
   long long step_base = 0, step = 0, step_end = 0;
   long long step_begin = -(long long)9e18;  // idles while step < step_begin (mrm_batch_delay_run)
@@ -156,8 +157,9 @@ struct Engine {
   Task* d_rtasks = nullptr;
   Task* d_ctasks = nullptr;
   int nrt = 0, nct = 0, rt_cap = 0, ct_cap = 0;
-  Task* d_ctasks2 = nullptr;  // column tasks of the register column kernel's runs (colreg.cuh)
-  int nct2 = 0, ct2_cap = 0;
+  // column tasks of the register column kernel's runs (colreg.cuh) of one and of two layers
+  Task* d_ctasks2[2] = {nullptr, nullptr};
+  int nct2[2] = {0, 0}, ct2_cap[2] = {0, 0};
   int rowv = 0, colv = 0, cpt = 0;  // row / column shapes (launch.h), columns per task (0: default)
   bool shape_forced = false;         // shapes set by the caller instead of tuned
   int force_rowv = 0, force_colv = 0, force_cpt = 0;
@@ -165,8 +167,10 @@ struct Engine {
   size_t smem_row[kRowSlots] = {0, 0, 0, 0, 0, 0};  // per launch slot (launch.h row_slot)
   int stage_cap[kRowSlots] = {0, 0, 0, 0, 0, 0};
   size_t smem_col = 0;
-  size_t smem_creg = 0;
-  int creg_tw_cap = 0, creg_blocks = 0;  // register column kernel: twiddle room, persistent blocks
+  // register column kernel for runs of one and two layers: shared memory,
+  // twiddle room, persistent blocks
+  size_t smem_creg[2] = {0, 0};
+  int creg_tw_cap[2] = {0, 0}, creg_blocks[2] = {0, 0};
   // the corrector with reductions always runs row shape 0 over one-row tasks,
   // so that the FP64 reductions do not depend on the tuned shapes
   Task* d_stasks = nullptr;
@@ -358,7 +362,7 @@ void engine_free(Engine* e) {
   dfree(e->d_runs);
   dfree(e->d_rtasks);
   dfree(e->d_ctasks);
-  dfree(e->d_ctasks2);
+  for (auto& p : e->d_ctasks2) dfree(p);
   dfree(e->d_stasks);
   dfree(e->d_part);
   dfree(e->d_stats);
@@ -400,8 +404,6 @@ int col_tile(int want) {
   return t;
 }
 int cols_per_task(const Engine* e, const mrm_gpu* r) { return col_tile(e->cpt > 0 ? e->cpt : default_cols(r)); }
-// shape of the register column kernel: the column shape index
-int creg_v(const Engine* e) { return std::min(std::max(e->colv, 0), kCregVariants - 1); }
 // cells per row and rows of the FFT source (the moving demag window, else the grid)
 int fnx(const mrm_gpu* r) { return r->wnx ? r->wnx : r->g.nx; }
 int fny(const mrm_gpu* r) { return r->wnx ? r->wny : r->g.ny; }
@@ -413,19 +415,52 @@ size_t specx_count(const mrm_gpu* r) {
 // (a windowed run's rows are segments of the grid's rows: one per task)
 int rows_per_task(const mrm_gpu* r, int rpb) { return r->wnx ? 1 : std::max(1, std::min(rpb, r->g.ny)); }
 
-// Runs whose column step is the register column kernel (colreg.cuh): FP32,
-// one layer, 256..1024-point columns.  Their tensor is stored in that
-// kernel's layout (tensor.cuh pack_tensor_creg_kernel).
-bool creg_run(const mrm_gpu* r) {
-  return r->g.precision == MRM_FP32 && r->nl == 1 && r->lgpy >= kCregMinLg && r->lgpy <= kCregMaxLg &&
-         !r->fft_big;
+// Runs whose column step is the register column kernel (colreg.cuh): FP32, one
+// layer with 64..1024-point columns or two with 512 or 1024 (shorter ones are
+// single runs whose blocks of six components crowd out the next kernel's early
+// start: 437 x 48 x 2 grains 54 us per step against 47 with the in-place kernel,
+// 500 x 75 x 2 60 against 54; 1024 x 256 x 2 190 against 235), with a symmetric
+// tensor: that kernel
+// keeps six components per layer pair (tensor.cuh pack_tensor_creg_kernel).
+// The SUL and head image terms make N_xz and N_zx differ; such a tensor keeps
+// its nine components and the in-place column kernel, which also takes the
+// other lengths and layer counts.
+bool creg_shape(const mrm_gpu* r) {
+  return r->g.precision == MRM_FP32 && r->nl <= 2 && r->lgpy >= (r->nl == 1 ? kCregMinLg : kCregMinLg2) &&
+         r->lgpy <= kCregMaxLg && !r->fft_big;
+}
+bool creg_run(const mrm_gpu* r) { return creg_shape(r) && r->tens_sym; }
+// shape of the register column kernel: the column shape index, if its groups
+// hold the longest columns
+int creg_v(const Engine* e) {
+  const int v = std::min(std::max(e->colv, 0), kCregVariants - 1);
+  bool fits = true, shorter = true;
+  for (auto* r : e->runs) {
+    if (!creg_run(r)) continue;
+    fits = fits && creg_pairs(r->lgpy, kCreg[v].group[r->nl - 1]) >= 1;
+    shorter = shorter && creg_pairs(r->lgpy, kCreg[kCregShort].group[r->nl - 1]) >= 1;
+  }
+  return v == 1 && shorter ? kCregShort : fits ? v : 0;
+}
+
+// shared memory of shape v for runs of nl layers: the staged M^ tile of a run
+// (the serial form reads the tiles in place), and the block's total
+int creg_stage_of(int v, const mrm_gpu* r) {
+  return kCreg[v].serial[r->nl - 1]
+             ? 0
+             : creg_stage_bytes(spec_col_stride(fny(r)), r->lgpy, kCreg[v].group[r->nl - 1], r->nl);
+}
+size_t creg_smem_of(int v, int nl, int tw_cap, int stage_bytes) {
+  return kCreg[v].serial[nl - 1] ? (size_t)cser_smem(tw_cap, kCreg[v].group[nl - 1])
+                                 : (size_t)creg_smem(tw_cap, kCreg[v].group[nl - 1], nl, stage_bytes);
 }
 
 size_t tensor_bytes(const mrm_gpu* r) {
   const size_t ph = r->px / 2 + 1, npair = (size_t)r->nl * r->nl;
   if (r->g.precision == MRM_FP64) return ph * npair * 9 * r->py * 2 * sizeof(double);
-  if (creg_run(r)) return ph * 6 * r->py * sizeof(float);
-  return ph * npair * 9 * tens_row_stride(r->py) * sizeof(float);
+  const size_t packed = ph * npair * 9 * tens_row_stride(r->py) * sizeof(float);
+  if (!creg_shape(r)) return packed;
+  return std::max(packed, (ph + 1) / 2 * creg_tensor_reals(r->lgpy, r->nl) * sizeof(float));
 }
 
 // row-kernel launch slots: kInit, kPred, kCorr, kCorr with reductions, kEval
@@ -435,6 +470,8 @@ constexpr int kSlotStage[kSlots] = {kInit, kPred, kCorr, kCorr, kEval, kPred};
 size_t row_static_bytes(int slot) {
   return ((slot == 3 || slot == 5) ? 32 * kNPart * sizeof(double) : sizeof(double)) + 128;
 }
+// static shared memory of the register column kernel (its tasks in flight) with margin
+constexpr size_t kCregStatic = 768;
 constexpr size_t kSmemPerSM = 228 * 1024;
 constexpr size_t kSmemReserved = 1024;  // per block
 
@@ -558,10 +595,9 @@ int validate_geom(const mrm_geom* g, std::string* errp, bool* big = nullptr) {
   const size_t rs = (f64 ? (size_t)row_fft_smem<double>(tmp.lgpx, 1) : (size_t)row_fft_smem<float>(tmp.lgpx, 1)) +
                     (size_t)(f64 ? head_table_bytes<double>(g->nx) : head_table_bytes<float>(g->nx));
   const size_t cs = f64 ? col_smem_of<double>(&tmp, 1, 0)
-                       : creg_run(&tmp) ? (size_t)creg_smem(col_tw_count(tmp.lgpy), kCreg[1].block,
-                                                            creg_stage_bytes(spec_col_stride(g->ny), 3))
+                       : creg_run(&tmp) ? creg_smem_of(0, tmp.nl, col_tw_count(tmp.lgpy), creg_stage_of(0, &tmp))
                                         : col_smem_of<float>(&tmp, 1, 0);
-  if (rs + row_static_bytes(3) > kMaxSmem || cs + 64 > kMaxSmem)
+  if (rs + row_static_bytes(3) > kMaxSmem || cs + kCregStatic > kMaxSmem)
     return set_err(errp, MRM_ERR_UNSUPPORTED, "FFT grid %d x %d x %d layers exceeds shared memory", px,
                    py, g->n_lay);
   return MRM_OK;
@@ -714,7 +750,8 @@ int plan_smem(Engine* e) {
   size_t fft = 16;
   int need[kSlots] = {0, 0, 0, 0, 0, 0}, least[kSlots] = {0, 0, 0, 0, 0, 0};
   size_t scol = 16;
-  int tw_cap = 0, stage_bytes = 0;
+  int tw_cap[2] = {0, 0}, stage_bytes[2] = {0, 0};
+  const int cv = creg_v(e);
   const RowPackCap pack = row_pack_cap<R>(e, rv.rpb);
   for (auto* r : e->runs) {
     if (r->lgpx > rv.lgmax)
@@ -728,8 +765,9 @@ int plan_smem(Engine* e) {
     }
     if (r->demag && r->tensor_ready) {
       if (creg_run(r)) {
-        tw_cap = std::max(tw_cap, col_tw_count(r->lgpy));
-        stage_bytes = std::max(stage_bytes, creg_stage_bytes(spec_col_stride(fny(r)), r->lgct));
+        int &tw = tw_cap[r->nl - 1], &sb = stage_bytes[r->nl - 1];
+        tw = std::max(tw, col_tw_count(r->lgpy));
+        sb = std::max(sb, creg_stage_of(cv, r));
       } else scol = std::max(scol, col_smem_of<R>(r, cols_per_task(e, r), col_variant<R>(e->colv).minb));
     }
   }
@@ -746,10 +784,12 @@ int plan_smem(Engine* e) {
   }
   if (scol + 64 > kMaxSmem) return set_err(errp, MRM_ERR_UNSUPPORTED, "column shape exceeds shared memory");
   e->smem_col = scol;
-  const size_t screg = tw_cap ? (size_t)creg_smem(tw_cap, kCreg[creg_v(e)].block, stage_bytes) : 16;
-  if (screg + 64 > kMaxSmem) return set_err(errp, MRM_ERR_UNSUPPORTED, "column shape exceeds shared memory");
-  e->smem_creg = screg;
-  e->creg_tw_cap = tw_cap;
+  for (int i = 0; i < 2; ++i) {
+    const size_t screg = tw_cap[i] ? creg_smem_of(cv, i + 1, tw_cap[i], stage_bytes[i]) : 16;
+    if (screg + kCregStatic > kMaxSmem) return set_err(errp, MRM_ERR_UNSUPPORTED, "column shape exceeds shared memory");
+    e->smem_creg[i] = screg;
+    e->creg_tw_cap[i] = tw_cap[i];
+  }
   CK(row_allow_smem<R>(e->rowv, e->smem_row));
   // the reductions launches (kPred of the single-stage integrator, kCorr):
   // row shape 0, one row per task
@@ -774,14 +814,15 @@ int plan_smem(Engine* e) {
     CK(row_allow_smem<R>(0, lim));
   }
   CK(col_allow_smem<R>(e->colv, e->smem_col));
-  e->creg_blocks = 0;
-  if (sizeof(R) == sizeof(float) && e->creg_tw_cap) {
-    CK(creg_allow_smem(creg_v(e), e->smem_creg));
+  for (int i = 0; i < 2; ++i) {
+    e->creg_blocks[i] = 0;
+    if (sizeof(R) != sizeof(float) || !e->creg_tw_cap[i]) continue;
+    CK(creg_allow_smem(cv, i + 1, e->smem_creg[i]));
     // persistent blocks: as many as stay resident
     int per_sm = 0, sms = 0;
-    CK(creg_occupancy(creg_v(e), e->smem_creg, &per_sm));
+    CK(creg_occupancy(cv, i + 1, e->smem_creg[i], &per_sm));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
-    e->creg_blocks = std::max(1, per_sm) * sms;
+    e->creg_blocks[i] = std::max(1, per_sm) * sms;
   }
   return MRM_OK;
 }
@@ -791,7 +832,8 @@ int build_tables(Engine* e) {
   std::string* errp = &e->err;
   const RowVariant rv = row_variant<R>(e->rowv);
   const RowPackCap pack = row_pack_cap<R>(e, rv.rpb);
-  std::vector<Task> rt, ct, ct2, stt;
+  std::vector<Task> rt, ct, ct2[2], stt;
+  const int cv = creg_v(e);
   for (size_t i = 0; i < e->runs.size(); ++i) {
     mrm_gpu* r = e->runs[i];
     r->slot = (int)i;
@@ -807,10 +849,10 @@ int build_tables(Engine* e) {
     if (r->demag && r->tensor_ready) {
       const int ph = r->px / 2 + 1;
       if (creg_run(r)) {
-        // a task per block of the register column kernel: block / (py/8) columns
-        const int cpt = creg_cols(r->lgpy, kCreg[creg_v(e)].block);
+        // a task is what a block of the register column kernel holds
+        const int cpt = 2 * creg_pairs(r->lgpy, kCreg[cv].group[r->nl - 1]);
         r->lgct = ilog2(col_tile(cpt));
-        for (int k = 0; k < ph; k += cpt) ct2.push_back(make_int4((int)i, k, std::min(cpt, ph - k), 0));
+        for (int k = 0; k < ph; k += cpt) ct2[r->nl - 1].push_back(make_int4((int)i, k, std::min(cpt, ph - k), 0));
       } else {
         const int cpt = cols_per_task(e, r);
         r->lgct = ilog2(cpt);
@@ -820,7 +862,7 @@ int build_tables(Engine* e) {
   }
   e->nrt = (int)rt.size();
   e->nct = (int)ct.size();
-  e->nct2 = (int)ct2.size();
+  for (int q = 0; q < 2; ++q) e->nct2[q] = (int)ct2[q].size();
   e->has_head = false;
   e->has_cubic = false;
   e->has_llb = false;
@@ -862,12 +904,13 @@ int build_tables(Engine* e) {
     int rc = dmalloc(errp, (void**)&e->d_ctasks, sizeof(Task) * e->ct_cap);
     if (rc) return rc;
   }
-  if (e->nct2 > e->ct2_cap) {
-    dfree(e->d_ctasks2);
-    e->ct2_cap = std::max(e->nct2, 2 * e->ct2_cap);
-    int rc = dmalloc(errp, (void**)&e->d_ctasks2, sizeof(Task) * e->ct2_cap);
-    if (rc) return rc;
-  }
+  for (int q = 0; q < 2; ++q)
+    if (e->nct2[q] > e->ct2_cap[q]) {
+      dfree(e->d_ctasks2[q]);
+      e->ct2_cap[q] = std::max(e->nct2[q], 2 * e->ct2_cap[q]);
+      int rc = dmalloc(errp, (void**)&e->d_ctasks2[q], sizeof(Task) * e->ct2_cap[q]);
+      if (rc) return rc;
+    }
   // the row tasks' records, then kMaxLayers frozen-grain records per run
   const int nr = (int)e->runs.size();
   const int npart = e->nst + nr * kMaxLayers;
@@ -890,7 +933,9 @@ int build_tables(Engine* e) {
   }
   if (e->nrt) CK(cudaMemcpyAsync(e->d_rtasks, rt.data(), sizeof(Task) * e->nrt, cudaMemcpyHostToDevice, e->st));
   if (e->nct) CK(cudaMemcpyAsync(e->d_ctasks, ct.data(), sizeof(Task) * e->nct, cudaMemcpyHostToDevice, e->st));
-  if (e->nct2) CK(cudaMemcpyAsync(e->d_ctasks2, ct2.data(), sizeof(Task) * e->nct2, cudaMemcpyHostToDevice, e->st));
+  for (int q = 0; q < 2; ++q)
+    if (e->nct2[q])
+      CK(cudaMemcpyAsync(e->d_ctasks2[q], ct2[q].data(), sizeof(Task) * e->nct2[q], cudaMemcpyHostToDevice, e->st));
   if (e->nst) CK(cudaMemcpyAsync(e->d_stasks, stt.data(), sizeof(Task) * e->nst, cudaMemcpyHostToDevice, e->st));
   CK(cudaStreamSynchronize(e->st));  // the host vectors are released on return
   int rc = plan_smem<R>(e);
@@ -928,11 +973,13 @@ cudaError_t launch_col_e(Engine* e, int istep, int flags, bool pdl = true) {
     cudaError_t ce = launch_col<R>(e->colv, a, istep, flags);
     if (ce != cudaSuccess) return ce;
   }
-  if (e->nct2) {
-    ColLaunch a{e->st, e->d_runs, e->d_ctasks2, e->d_tw, e->d_err, e->nct2, e->smem_creg, pdl};
-    a.blocks = e->creg_blocks;
-    a.tw_cap = e->creg_tw_cap;
-    return launch_creg(creg_v(e), a, istep, flags);
+  for (int q = 0; q < 2; ++q) {
+    if (!e->nct2[q]) continue;
+    ColLaunch a{e->st, e->d_runs, e->d_ctasks2[q], e->d_tw, e->d_err, e->nct2[q], e->smem_creg[q], pdl};
+    a.blocks = e->creg_blocks[q];
+    a.tw_cap = e->creg_tw_cap[q];
+    const cudaError_t ce = launch_creg(creg_v(e), q + 1, a, istep, flags);
+    if (ce != cudaSuccess) return ce;
   }
   return cudaSuccess;
 }
@@ -1800,14 +1847,14 @@ cudaError_t launch_tensor_real(double* d_n2d, const PairGeom* d_pg, int npair, i
 }
 
 // Temporaries of a tensor build: the real tensor, its spectrum, FP64
-// twiddles, the pair geometries and the two diagnostic maxima.
+// twiddles, the pair geometries and the diagnostic maxima.
 struct TensorScratch : Scratch {
   size_t n2d, spec, tw, pg, mx;
   TensorScratch(const mrm_gpu* r, bool spectrum) {
     const size_t npair = (size_t)r->nl * r->nl, planes = npair * 9;
     n2d = take(sizeof(double) * planes * r->px * r->py);
     pg = take(sizeof(PairGeom) * npair);
-    mx = take(2 * sizeof(unsigned long long));
+    mx = take(3 * sizeof(unsigned long long));
     spec = spectrum ? take(sizeof(double) * 2 * planes * r->py * (r->px / 2 + 1)) : 0;
     tw = spectrum ? take(sizeof(double) * 2 * kTwN) : 0;
   }
@@ -1843,7 +1890,7 @@ int tensor_spectrum(mrm_gpu* r, const TensorScratch& w) {
   const Cx<double>* tw64 = w.at<Cx<double>>(w.tw);
   unsigned long long* d_mx = w.at<unsigned long long>(w.mx);
   CK(h2d(w.at<double>(w.tw), twiddles64().data(), sizeof(double) * 2 * kTwN));
-  CK(cudaMemsetAsync(d_mx, 0, 2 * sizeof(unsigned long long), e->st));
+  CK(cudaMemsetAsync(d_mx, 0, 3 * sizeof(unsigned long long), e->st));
   const int M = r->px / 2;
   // two shared buffers of one padded-stride sequence each (fft.cuh)
   size_t s1 = 2 * (size_t)pad_stride(M) * sizeof(Cx<double>), s2 = 2 * (size_t)pad_stride(r->py) * sizeof(Cx<double>);
@@ -1853,29 +1900,40 @@ int tensor_spectrum(mrm_gpu* r, const TensorScratch& w) {
   CK(cudaGetLastError());
   c2c_cols_f64<<<planes * ph, 256, s2, e->st>>>(d_spec, r->lgpy, ph, tw64);
   CK(cudaGetLastError());
+  const bool was_creg = creg_run(r);
+  // the maxima: wrong-parity residue, kept part, difference from the transpose
+  double mx[3];
+  auto read_maxima = [&]() -> cudaError_t {
+    cudaError_t ce = cudaGetLastError();
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(mx, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, e->st);
+    return ce == cudaSuccess ? cudaStreamSynchronize(e->st) : ce;
+  };
+  bool packed = false;
   if (e->prec == MRM_FP64) {
     const long long total = (long long)ph * npair * 9 * r->py;
     pack_tensor_full_kernel<<<(unsigned)((total + 255) / 256), 256, 0, e->st>>>(
         d_spec, static_cast<Cx<double>*>(r->tens), npair, r->py, ph, d_mx, d_mx + 1);
-  } else if (creg_run(r)) {
-    const long long total = (long long)ph * 6 * r->py;
+    CK(read_maxima());
+    packed = true;
+  } else if (creg_shape(r)) {
+    const long long total = (long long)((ph + 1) / 2) * (long long)creg_tensor_reals(r->lgpy, r->nl);
     pack_tensor_creg_kernel<<<(unsigned)((total + 255) / 256), 256, 0, e->st>>>(
-        d_spec, static_cast<float*>(r->tens), r->lgpy, ph, d_mx, d_mx + 1);
-  } else {
+        d_spec, static_cast<float*>(r->tens), npair, r->lgpy, ph, d_mx);
+    CK(read_maxima());
+    // symmetric to the rounding of the FP32 store (4 ulp of the largest value)
+    r->tens_sym = packed = !(mx[2] > 2.4e-7 * mx[1]);
+  }
+  if (!packed) {
+    CK(cudaMemsetAsync(d_mx, 0, 3 * sizeof(unsigned long long), e->st));
     const long long total = (long long)ph * npair * 9 * pyh;
     pack_tensor_kernel<float><<<(unsigned)((total + 255) / 256), 256, 0, e->st>>>(
-        d_spec, static_cast<float*>(r->tens), npair, r->py, ph,
-        tens_row_stride(r->py), d_mx, d_mx + 1);
+        d_spec, static_cast<float*>(r->tens), npair, r->py, ph, tens_row_stride(r->py), d_mx, d_mx + 1);
+    CK(read_maxima());
   }
-  CK(cudaGetLastError());
-  unsigned long long hm[2];
-  CK(cudaMemcpyAsync(hm, d_mx, sizeof(hm), cudaMemcpyDeviceToHost, e->st));
-  CK(cudaStreamSynchronize(e->st));
-  double dres, dkept;
-  std::memcpy(&dres, &hm[0], 8);
-  std::memcpy(&dkept, &hm[1], 8);
-  r->tensor_resid = dres;
-  r->tensor_kept = dkept;
+  r->tensor_resid = creg_run(r) ? std::max(mx[0], mx[2]) : mx[0];
+  r->tensor_kept = mx[1];
+  // (tasks and tiles follow the column kernel of the run)
+  if (was_creg != creg_run(r)) e->tables_dirty = true;
   // (the tasks list the runs with a tensor: a rebuilt one changes none of them)
   if (!r->tensor_ready) e->tables_dirty = true;
   r->tensor_ready = true;
@@ -2235,6 +2293,7 @@ int mrm_gpu_copy_tensor(mrm_gpu* dst, const mrm_gpu* src) {
   dst->tensor_ready = true;
   dst->tensor_resid = src->tensor_resid;
   dst->tensor_kept = src->tensor_kept;
+  dst->tens_sym = src->tens_sym;
   dst->spec_valid = false;
   dst->eng->tables_dirty = true;
   dst->eng->desc_dirty = true;
@@ -3519,7 +3578,8 @@ static int occ_t(Engine* e, int* out2) {
   if (!e->tables_dirty) {
     CK(row_occupancy<R>(e->rowv, kPred, e->smem_row[1], &a));
     // the column kernel of most of the batch's column tasks
-    if (e->nct2 > e->nct) CK(creg_occupancy(creg_v(e), e->smem_creg, &b));
+    const int q = e->nct2[1] > e->nct2[0] ? 1 : 0;
+    if (e->nct2[q] > e->nct) CK(creg_occupancy(creg_v(e), q + 1, e->smem_creg[q], &b));
     else CK(col_occupancy<R>(e->colv, e->smem_col, &b));
   }
   out2[0] = a;
@@ -3661,7 +3721,7 @@ int noalloc_setup(int dev, std::string* errp, unsigned char** base) {
   for (int q = 0; q < kSlots; ++q) lim[q] = (size_t)optin - row_static_bytes(q);
   CK(row_allow_smem<float>(0, lim));
   CK(col_allow_smem<float>(0, (size_t)optin - 64));
-  CK(creg_allow_smem(0, (size_t)optin - 64));
+  for (int nl = 1; nl <= 2; ++nl) CK(creg_allow_smem(0, nl, (size_t)optin - kCregStatic));
   cudaFuncAttributes fa;
   CK(cudaFuncGetAttributes(&fa, noalloc_pack_kernel));
   CK(cudaFuncGetAttributes(&fa, noalloc_unpack_kernel));
@@ -3689,7 +3749,7 @@ int mrm_gpu_demag_noalloc(mrm_gpu* h, const float* m, float* hdemag, void* strea
   const int nl = h->nl, ny = h->g.ny, ph = h->px / 2 + 1;
   const int rpt = 1, nrt = nl * ny;  // one row per task (row shape 0)
   const bool creg = creg_run(h);
-  const int cpt = creg ? creg_cols(h->lgpy, kCreg[0].block) : col_tile(default_cols(h)), nct = (ph + cpt - 1) / cpt;
+  const int cpt = creg ? 2 * creg_pairs(h->lgpy, kCreg[0].group[nl - 1]) : col_tile(default_cols(h)), nct = (ph + cpt - 1) / cpt;
   const NoAllocLayout lay = noalloc_layout(h, nrt, nct);
   if (lay.total > kNoAllocBytes)
     return set_err(errp, MRM_ERR_UNSUPPORTED,
@@ -3713,7 +3773,7 @@ int mrm_gpu_demag_noalloc(mrm_gpu* h, const float* m, float* hdemag, void* strea
   d.demag = 1;
   d.row_task0 = 0;
   d.nrow_tasks = nrt;
-  d.lgct = ilog2(cpt);
+  d.lgct = ilog2(col_tile(cpt));
   d.specx = reinterpret_cast<Cx<float>*>(base + lay.specx);
   d.spech = reinterpret_cast<Cx<float>*>(base + lay.spech);
   V4<float>* sm = reinterpret_cast<V4<float>*>(base + lay.m);
@@ -3749,11 +3809,10 @@ int mrm_gpu_demag_noalloc(mrm_gpu* h, const float* m, float* hdemag, void* strea
                        0, kFlagForce));
   if (creg) {
     ColLaunch a{st, desc, ct, e->d_tw, e->d_err, nct,
-                (size_t)creg_smem(col_tw_count(h->lgpy), kCreg[0].block,
-                                  creg_stage_bytes(spec_col_stride(ny), ilog2(cpt))),
+                creg_smem_of(0, nl, col_tw_count(h->lgpy), creg_stage_of(0, h)),
                 true};
     a.tw_cap = col_tw_count(h->lgpy);
-    CK(launch_creg(0, a, 0, kFlagForce));
+    CK(launch_creg(0, nl, a, 0, kFlagForce));
   }
   else
     CK(launch_col<float>(0, ColLaunch{st, desc, ct, e->d_tw, e->d_err, nct, col_smem_of<float>(h, cpt, col_variant<float>(0).minb), true}, 0,

@@ -383,38 +383,46 @@ __global__ void pack_tensor_kernel(const Cx<double>* __restrict__ spec, R* __res
   block_max2(disc, fabs(keep), resid, kept);
 }
 
-// spectrum [0][9][py][ph] (FP64, one layer) -> tens[k][6][py] floats for the
-// register column kernel (colreg.cuh): components xx, yy, zz, xy, xz, yz (the
-// tensor is symmetric: yx, zx, zy are xy, xz, yz) at the positions of the
-// column transform's digit-reversed order (element p holds k_y = ip_freq(p)),
-// the sign of the odd components for k_y > py/2 folded in.  The residue adds
-// any difference between a component and its transpose.
-__global__ void pack_tensor_creg_kernel(const Cx<double>* __restrict__ spec, float* __restrict__ tens, int lgpy,
-                                        int ph, unsigned long long* resid, unsigned long long* kept) {
+// spectrum [pair][9][py][ph] (FP64) -> the register column kernel's tensor
+// (colreg.cuh): floats [column pair][pair of layers][6][j < 4][t < py/8][h < 2][column],
+// components xx, yy, zz, xy, xz, yz (yx, zx, zy taken as xy, xz, yz) at
+// position 8t + 2j + h of the column transform's digit-reversed order (element
+// p holds k_y = ip_freq(p)), the sign of the odd components for k_y > py/2
+// folded in, zero for the partner of a last odd column.  mx: wrong-parity
+// residue, kept part, largest difference between a component and its transpose.
+__global__ void pack_tensor_creg_kernel(const Cx<double>* __restrict__ spec, float* __restrict__ tens, int npair,
+                                        int lgpy, int ph, unsigned long long* mx) {
   const int py = 1 << lgpy;
-  const long long total = (long long)ph * 6 * py;
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double keep = 0.0, disc = 0.0;
-  if (gid < total) {
-    const int p = (int)(gid % py);
-    const int c6 = (int)((gid / py) % 6);
-    const int k = (int)(gid / ((long long)6 * py));
-    const int ky = ip_freq(p, lgpy);
+  const long long per = (long long)npair * 6 * 2 * py;
+  double keep = 0.0, disc = 0.0, asym = 0.0;
+  if (gid < (ph + 1) / 2 * per) {
+    const int col = (int)(gid & 1), h = (int)(gid >> 1) & 1;
+    const int t = (int)(gid >> 2) & (py / 8 - 1), j = (int)(gid >> (lgpy - 1)) & 3;
+    const int r = (int)((gid % per) >> (lgpy + 1)), c6 = r % 6, pair = r / 6;
+    const int k = 2 * (int)(gid / per) + col;
+    const int ky = ip_freq(8 * t + 2 * j + h, lgpy);
     const bool upper = ky > py / 2;
     const int kyh = upper ? py - ky : ky;
     constexpr int kComp[6] = {0, 4, 8, 1, 2, 5};   // xx yy zz xy xz yz
     constexpr int kTrans[6] = {0, 4, 8, 3, 6, 7};  // their transposes
-    const int c = kComp[c6];
-    parity_parts(spec + (long long)c * py * ph, c, kyh, k, py, ph, &keep, &disc);
-    if (kTrans[c6] != c) {
-      double kt, dt;
-      parity_parts(spec + (long long)kTrans[c6] * py * ph, kTrans[c6], kyh, k, py, ph, &kt, &dt);
-      disc = fmax(disc, fmax(dt, fabs(kt - keep)));
+    const int c = kComp[c6], ct = kTrans[c6];
+    if (k < ph) {
+      const Cx<double>* S = spec + (long long)pair * 9 * py * ph;
+      parity_parts(S + (long long)c * py * ph, c, kyh, k, py, ph, &keep, &disc);
+      if (ct != c) {
+        double kt, dt;
+        parity_parts(S + (long long)ct * py * ph, ct, kyh, k, py, ph, &kt, &dt);
+        disc = fmax(disc, dt);
+        asym = fabs(kt - keep);
+      }
     }
     const bool odd = (kOddMask >> c) & 1;
     tens[gid] = (float)((odd && upper) ? -keep : keep);
   }
-  block_max2(disc, fabs(keep), resid, kept);
+  block_max2(disc, fabs(keep), mx, mx + 1);
+  __syncthreads();
+  block_max2(asym, 0.0, mx + 2, mx + 1);
 }
 
 // spectrum [pair][9][py][ph] -> tens[k][pair][c][ky] complex, unchanged (FP64 runs)
