@@ -204,7 +204,8 @@ struct alignas(16) RunDev {
   // arrays; frz: the run's first stats record of the frozen grains (-1: none)
   int gnx, gny, wi0, wj0, frz;
   const R* tens;           // tensor spectrum: FP32 packed [px/2+1][nl*nl][9][pyhs] reals,
-                           // FP64 full [px/2+1][nl*nl][9][py] complex
+                           // FP64 full [px/2+1][nl*nl][9][py] complex, each column in the
+                           // digit-reversed order of the column transform
   LayerDev<R> L[kMaxLayers];
 };
 

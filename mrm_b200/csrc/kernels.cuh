@@ -1890,9 +1890,20 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
 // of column c in plane p sits at p*col_plane(py, lgct) + ((j + j/8) << lgct) + c:
 // one pad row every 8 rows keeps the 8-element butterflies of the last forward
 // (and first inverse) pass on distinct banks.
-constexpr int kTensSliceBytes = 48 * 1024;
+// The tensor of a task's columns is staged in shared memory, by a bulk copy ahead
+// of the dependency wait, up to 48 KB in FP32 and 80 KB in FP64 (one 512-point
+// column's nine complex components, 74 KB): the product then waits for no
+// global load.  (256 x 256 FP64 run, with the FP64 tensor in the order of the
+// transform's positions so that a warp reads consecutive values: 63.1 -> 49.5 us
+// per step; 64 x 64: 27.7 -> 26.7.)
 template <typename R>
-MRM_HD bool tens_slice_fits(int reals) { return (size_t)reals * sizeof(R) <= (size_t)kTensSliceBytes; }
+MRM_HD int tens_slice_reals(int nc, int npair, int py, int pyhs) {
+  return nc * npair * 9 * (sizeof(R) == sizeof(float) ? pyhs : 2 * py);
+}
+template <typename R>
+MRM_HD bool tens_slice_fits(int reals) {
+  return (size_t)reals * sizeof(R) <= (size_t)(sizeof(R) == sizeof(float) ? 48 : 80) * 1024;
+}
 
 MRM_HD constexpr int col_plane(int py, int lgct) { return (py + (py >> 3)) << lgct; }
 // complex values of one column buffer (even: what follows stays 16-byte aligned)
@@ -1917,13 +1928,14 @@ MRM_D void col_product(const RunDev<R>& rd, Cx<R>* A, Cx<R>* O, const R* Ts, boo
   (void)tens_len;
   (void)err;
   // 3 outputs of layer ko at one position from the inputs of every layer
-  auto mac = [&](int c, int ky, int ko, const Cx<R>* x, int xstride, Cx<R> h[3]) {
+  auto mac = [&](int c, int p, int ko, const Cx<R>* x, int xstride, Cx<R> h[3]) {
     h[0] = h[1] = h[2] = Cx<R>{(R)0, (R)0};
     for (int ks = 0; ks < nl; ++ks) {
       Cx<R> xm[3];
 #pragma unroll
       for (int b = 0; b < 3; ++b) xm[b] = x[(size_t)(ks * 3 + b) * xstride];
       if constexpr (PACKED) {
+        const int ky = ip_freq(p, lgpy);
         const bool upper = ky > (py >> 1);
         const int kyh = upper ? py - ky : ky;
         const size_t off = ((size_t)c * npair + ks * nl + ko) * 9 * pyhs;
@@ -1946,10 +1958,12 @@ MRM_D void col_product(const RunDev<R>& rd, Cx<R>* A, Cx<R>* O, const R* Ts, boo
             else h[a] = cadd(h[a], cscale(xm[b], v));
           }
       } else {
-        const Cx<R>* Tc = reinterpret_cast<const Cx<R>*>(rd.tens) + ((size_t)(k0 + c) * npair + ks * nl + ko) * 9 * py;
+        const size_t off = ((size_t)c * npair + ks * nl + ko) * 9 * py + p;
+        const Cx<R>* Tc = tsm ? reinterpret_cast<const Cx<R>*>(Ts) + off
+                              : reinterpret_cast<const Cx<R>*>(rd.tens) + (size_t)k0 * npair * 9 * py + off;
         Cx<R> tv[9];
 #pragma unroll
-        for (int cc = 0; cc < 9; ++cc) tv[cc] = Tc[cc * py + ky];
+        for (int cc = 0; cc < 9; ++cc) tv[cc] = Tc[cc * py];
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -1961,14 +1975,13 @@ MRM_D void col_product(const RunDev<R>& rd, Cx<R>* A, Cx<R>* O, const R* Ts, boo
     for (int idx = threadIdx.x; idx < (py << lgct); idx += BLOCK) {
       const int c = idx & (T - 1), p = idx >> lgct;
       if (c >= nc) continue;
-      const int ky = ip_freq(p, lgpy);
       const int at = ((p + (p >> 3)) << lgct) + c;
       Cx<R> xin[3 * NLC];
 #pragma unroll
       for (int i = 0; i < 3 * NLC; ++i) xin[i] = A[(size_t)i * plane + at];
       Cx<R> h[NLC][3];
 #pragma unroll
-      for (int ko = 0; ko < NLC; ++ko) mac(c, ky, ko, xin, 1, h[ko]);
+      for (int ko = 0; ko < NLC; ++ko) mac(c, p, ko, xin, 1, h[ko]);
 #pragma unroll
       for (int ko = 0; ko < NLC; ++ko)
 #pragma unroll
@@ -1978,10 +1991,9 @@ MRM_D void col_product(const RunDev<R>& rd, Cx<R>* A, Cx<R>* O, const R* Ts, boo
     for (int idx = threadIdx.x; idx < (nl * py) << lgct; idx += BLOCK) {
       const int c = idx & (T - 1), p = (idx >> lgct) & (py - 1), ko = idx >> (lgct + lgpy);
       if (c >= nc) continue;
-      const int ky = ip_freq(p, lgpy);
       const int at = ((p + (p >> 3)) << lgct) + c;
       Cx<R> h[3];
-      mac(c, ky, ko, A + at, plane, h);
+      mac(c, p, ko, A + at, plane, h);
 #pragma unroll
       for (int a = 0; a < 3; ++a) O[(size_t)(ko * 3 + a) * plane + at] = h[a];
     }
@@ -2077,12 +2089,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) col_kernel(const RunDev<R>* __res
   const int ntw = col_tw_count(lgpy);
   Cx<R>* A = tws + ntw;
   const int npair = nl * nl;
-  const int tslice = nc * npair * 9 * pyhs;  // reals
+  const int tslice = tens_slice_reals<R>(nc, npair, py, pyhs);  // reals
   R* Ts = reinterpret_cast<R*>(A + (nl > 2 ? 2 : 1) * col_buf_count(py, lgct, nl * 3));
   // the slice is staged only where the launch's shared memory holds it (the
   // host leaves it out where it would cost resident blocks, and a smaller last
   // task may fit where the largest does not)
-  const bool tsm = PACKED && tens_slice_fits<R>(tslice) &&
+  const bool tsm = tens_slice_fits<R>(tslice) &&
                    (long long)(reinterpret_cast<unsigned char*>(Ts) - smem_raw) + (long long)tslice * sizeof(R) <=
                        (long long)dynamic_smem_bytes();
   MRM_CHECK(k0 >= 0 && nc >= 1 && k0 + nc <= ph && (k0 & ((1 << lgct) - 1)) == 0 && nc <= (1 << lgct), 500, k0);
@@ -2093,7 +2105,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) col_kernel(const RunDev<R>* __res
     mbar_fence_init();
   }
   __syncthreads();
-  // static inputs: twiddles and this task's packed tensor slice (columns k0.. are contiguous)
+  // static inputs: twiddles and this task's tensor slice (columns k0.. are contiguous)
   auto copy = [&](uint64_t* bar, void* dst, const void* src, long long src_off_bytes, long long src_len_bytes,
                   int bytes, int code) {
 #ifdef MRM_CHECKS
@@ -2112,8 +2124,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) col_kernel(const RunDev<R>* __res
   if (threadIdx.x == 0) {
     copy(&bars[0], tws, twg + rd.tw_col, rd.tw_col * cb, (long long)tw_table_size() * cb, ntw * (int)cb, 400);
     if (tsm) {
-      const long long off = (long long)k0 * npair * 9 * pyhs;
-      copy(&bars[0], Ts, rd.tens + off, off * (long long)sizeof(R), (long long)ph * npair * 9 * pyhs * sizeof(R),
+      const long long per = tens_slice_reals<R>(1, npair, py, pyhs), off = (long long)k0 * per;
+      copy(&bars[0], Ts, rd.tens + off, off * (long long)sizeof(R), (long long)ph * per * sizeof(R),
            tslice * (int)sizeof(R), 410);
     }
     mbar_arrive(&bars[0]);

@@ -548,8 +548,8 @@ size_t row_fixed_smem(const mrm_gpu* r, int rpb) {
 template <typename R>
 size_t col_smem_of(const mrm_gpu* r, int nc, int minb) {
   const size_t b = col_fft_smem<R>(r->lgpy, ilog2(nc), r->nl * 3);
-  if (sizeof(R) != sizeof(float) || minb <= 0) return b;
-  const int reals = nc * r->nl * r->nl * 9 * tens_row_stride(r->py);
+  if (minb <= 0) return b;
+  const int reals = tens_slice_reals<R>(nc, r->nl * r->nl, r->py, tens_row_stride(r->py));
   if (!tens_slice_fits<R>(reals)) return b;
   const size_t with = b + (size_t)reals * sizeof(R);
   auto resident = [](size_t bytes) { return (int)(kSmemPerSM / (bytes + kSmemReserved)); };
@@ -1912,7 +1912,7 @@ int tensor_spectrum(mrm_gpu* r, const TensorScratch& w) {
   if (e->prec == MRM_FP64) {
     const long long total = (long long)ph * npair * 9 * r->py;
     pack_tensor_full_kernel<<<(unsigned)((total + 255) / 256), 256, 0, e->st>>>(
-        d_spec, static_cast<Cx<double>*>(r->tens), npair, r->py, ph, d_mx, d_mx + 1);
+        d_spec, static_cast<Cx<double>*>(r->tens), npair, r->lgpy, ph, d_mx, d_mx + 1);
     CK(read_maxima());
     packed = true;
   } else if (creg_shape(r)) {

@@ -425,15 +425,18 @@ __global__ void pack_tensor_creg_kernel(const Cx<double>* __restrict__ spec, flo
   block_max2(asym, 0.0, mx + 2, mx + 1);
 }
 
-// spectrum [pair][9][py][ph] -> tens[k][pair][c][ky] complex, unchanged (FP64 runs)
+// spectrum [pair][9][py][ph] -> tens[k][pair][c][p] complex (FP64 runs), position
+// p of the column transform's digit-reversed order holding k_y = ip_freq(p), so
+// the product reads consecutive values
 __global__ void pack_tensor_full_kernel(const Cx<double>* __restrict__ spec, Cx<double>* __restrict__ tens,
-                                        int npair, int py, int ph, unsigned long long* resid,
+                                        int npair, int lgpy, int ph, unsigned long long* resid,
                                         unsigned long long* kept) {
+  const int py = 1 << lgpy;
   const long long total = (long long)ph * npair * 9 * py;
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double keep = 0.0, disc = 0.0;
   if (gid < total) {
-    const int ky = (int)(gid % py);
+    const int ky = ip_freq((int)(gid % py), lgpy);
     long long r = gid / py;
     const int c = (int)(r % 9);
     r /= 9;
