@@ -19,7 +19,7 @@ LIB = os.path.join(HERE, "libmrm_gpu.so")
 OBJ = os.path.join(HERE, "_build")
 # longest compiles first (the pool takes them in this order)
 SOURCES = ([f"csrc/k_row_f32_v{v}_g{g}.cu" for g in (2, 1, 0) for v in range(5)] +
-           [f"csrc/k_creg_v{v}.cu" for v in range(4)] + [f"csrc/k_row_f64_v{v}.cu" for v in range(3)] +
+           [f"csrc/k_creg_v{v}.cu" for v in range(5)] + [f"csrc/k_row_f64_v{v}.cu" for v in range(3)] +
            [f"csrc/k_col_f32_v{v}.cu" for v in range(3)] + [f"csrc/k_col_f64_v{v}.cu" for v in range(2)] +
            ["csrc/mrm_gpu.cu", "csrc/k_col.cu", "csrc/k_row_split.cu"])
 HEADERS = ["csrc/common.cuh", "csrc/fft.cuh", "csrc/kernels.cuh", "csrc/philox.cuh", "csrc/tensor.cuh",

@@ -305,9 +305,11 @@ MRM_D void creg_stage(float4* __restrict__ buf, int t, const float4* __restrict_
 // those of one layer are loaded ahead of the task's transforms, which cover
 // their latency (the tensor never changes: the first task's come in before the
 // previous kernel has finished), further layers' as the product goes.
-template <int LGN, int G, int NL>
+// AHEAD: the pieces loaded ahead (both of one layer where the launch bounds
+// leave a thread the registers: at most 384 threads per SM).
+template <int LGN, int G, int NL, int AHEAD>
 struct CregTens {
-  static constexpr int PIECES = 2 * NL, AHEAD = NL == 1 && G <= 64 ? 2 : 1;
+  static constexpr int PIECES = 2 * NL;
   ulonglong2 v[PIECES][3][2];
   const ulonglong2* tn;
   // k0 < 0: nothing to load
@@ -337,8 +339,8 @@ struct CregTens {
 // inverse transforms.  stg: the task's M^ tiles staged in shared memory
 // ([plane][tile][nys][T]); xb: the exchange buffers; `staged_read` runs once
 // every thread has its stage-0 elements in registers.
-template <int LGN, int G, int NL, bool HALF, class AFTER>
-MRM_D void creg_body(const RunDev<float>& rd, int k0, int nc, CregTens<LGN, G, NL>& tens,
+template <int LGN, int G, int NL, int AHEAD, bool HALF, class AFTER>
+MRM_D void creg_body(const RunDev<float>& rd, int k0, int nc, CregTens<LGN, G, NL, AHEAD>& tens,
                      const float4* __restrict__ tw, const Cx<float>* __restrict__ stg, float4* __restrict__ xb,
                      const AFTER& staged_read) {
   using P = RegPlan<LGN>;
@@ -388,7 +390,7 @@ MRM_D void creg_body(const RunDev<float>& rd, int k0, int nc, CregTens<LGN, G, N
 #pragma unroll
   for (int hs = 0; hs < 2 * NL; ++hs) {
     const int half = hs / NL, s = hs - half * NL;
-    if (hs + CregTens<LGN, G, NL>::AHEAD < 2 * NL) tens.load(hs + CregTens<LGN, G, NL>::AHEAD);
+    if (hs + AHEAD < 2 * NL) tens.load(hs + AHEAD);
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       const float4* m = xb + (s * 3 + b) * SEQ + at8 + 4 * half * PR;
@@ -556,12 +558,12 @@ struct CregLoop {
 
 // The block's tasks from the current one on for as long as they have this
 // column length and padding (the current one does); false: a copy did not land.
-template <int LGN, int G, int NL, bool HALF>
+template <int LGN, int G, int NL, int AHEAD, bool HALF>
 MRM_D bool creg_run(CregLoop& c, const float4* tw, float4* xb) {
   if constexpr ((1 << (LGN - 3)) <= G) {
     while (true) {
       const RunDev<float>& rd = c.rd(c.r);
-      CregTens<LGN, G, NL> tens;
+      CregTens<LGN, G, NL, AHEAD> tens;
       tens.start(rd, rd.active && rd.demag ? c.ct->cols[c.r].x : -1, c.ct->cols[c.r].y);
       c.begin();
       if (!c.landed()) return false;
@@ -570,7 +572,7 @@ MRM_D bool creg_run(CregLoop& c, const float4* tw, float4* xb) {
         __syncthreads();
         c.issue_next();
       } else {
-        creg_body<LGN, G, NL, HALF>(rd, kc.x, kc.y, tens, tw, c.stg, xb, [&]() { c.issue_next(); });
+        creg_body<LGN, G, NL, AHEAD, HALF>(rd, kc.x, kc.y, tens, tw, c.stg, xb, [&]() { c.issue_next(); });
       }
       c.advance();
       if (c.i >= c.ntasks) return true;
@@ -654,8 +656,8 @@ __global__ void __launch_bounds__(3 * NL * G, MINB)
     }
     const bool half = rd.py >= 2 * rd.ny;
     auto go = [&](auto lg) {
-      constexpr int LGN = decltype(lg)::value;
-      ok = half ? creg_run<LGN, G, NL, true>(c, tws, xb) : creg_run<LGN, G, NL, false>(c, tws, xb);
+      constexpr int LGN = decltype(lg)::value, AHEAD = NL == 1 && 3 * NL * G * MINB <= 384 ? 2 : 1;
+      ok = half ? creg_run<LGN, G, NL, AHEAD, true>(c, tws, xb) : creg_run<LGN, G, NL, AHEAD, false>(c, tws, xb);
     };
     if constexpr (NL == 1) {
       switch (lgpy) {

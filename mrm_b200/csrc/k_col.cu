@@ -184,6 +184,7 @@ static const CregOps* creg_ops_of(int v, int nl) {
     case 1: return &creg_ops<1>();
     case 2: return &creg_ops<2>();
     case 3: return &creg_ops<3>();
+    case 4: return &creg_ops<4>();
     default: return nullptr;
   }
 }

@@ -49,15 +49,20 @@ struct CregVariant {
   int group[2], minb[2];
   bool serial[2];
 };
-constexpr int kCregVariants = 3, kCregShapes = 4;
+constexpr int kCregVariants = 3, kCregShapes = 5;
 constexpr CregVariant kCreg[kCregShapes] = {{{128, 128}, {2, 1}, {false, false}},
                                             {{64, 64}, {2, 2}, {false, false}},
                                             {{128, 64}, {3, 2}, {true, false}},
-                                            {{32, 64}, {2, 2}, {false, false}}};
+                                            {{32, 64}, {2, 2}, {false, false}},
+                                            {{128, 128}, {1, 1}, {false, false}}};
 // column shape 1 where no column is longer than its groups hold: half the
 // columns to a block spread a single run's few tasks over twice the blocks
 // (200 x 75 grains: 36.0 -> 34.6 us per step)
 constexpr int kCregShort = 3;
+// column shape 1 where a column is longer than its groups hold: shape 0's
+// groups with the registers of one block per SM, which hold the tensor loaded
+// ahead (91 x 505 grains: 61 -> 48 us per step)
+constexpr int kCregLong = 4;
 constexpr int creg_block(int v, int nl) { return kCreg[v].group[nl - 1] * (kCreg[v].serial[nl - 1] ? 1 : 3 * nl); }
 
 struct RowLaunch;

@@ -430,8 +430,9 @@ bool creg_shape(const mrm_gpu* r) {
          r->lgpy <= kCregMaxLg && !r->fft_big;
 }
 bool creg_run(const mrm_gpu* r) { return creg_shape(r) && r->tens_sym; }
-// shape of the register column kernel: the column shape index, if its groups
-// hold the longest columns
+// shape of the register column kernel: the column shape index, with the group
+// size of shape 1 (a single run's, registers before resident blocks) by the
+// longest columns
 int creg_v(const Engine* e) {
   const int v = std::min(std::max(e->colv, 0), kCregVariants - 1);
   bool fits = true, shorter = true;
@@ -440,7 +441,7 @@ int creg_v(const Engine* e) {
     fits = fits && creg_pairs(r->lgpy, kCreg[v].group[r->nl - 1]) >= 1;
     shorter = shorter && creg_pairs(r->lgpy, kCreg[kCregShort].group[r->nl - 1]) >= 1;
   }
-  return v == 1 && shorter ? kCregShort : fits ? v : 0;
+  return v == 1 ? (shorter ? kCregShort : fits ? 1 : kCregLong) : fits ? v : 0;
 }
 
 // shared memory of shape v for runs of nl layers: the staged M^ tile of a run
