@@ -59,10 +59,10 @@ WORKLOAD = ("batched {b} x 65,536-grain M(H) ramp realisations, T=300 K, FP32, "
 
 # DRAM traffic per launch of each kernel in bytes per grain of the launch:
 # dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of the
-# headline batch (32 x 65,536 grains, row shape 1, the register column kernel
-# {128 threads, 4 blocks/SM}, one column per task), divided by its grains; a
-# kernel change calls for a new capture
-NCU_TRAFFIC_BYTES_PER_GRAIN = {"row_pred": 141.0, "col": 35.7, "row_corr": 164.4}
+# headline batch (32 x 65,536 grains, row shape 3, the register column kernel
+# in turn {128 threads, 3 blocks/SM}, one column per task), divided by its
+# grains; a kernel change calls for a new capture
+NCU_TRAFFIC_BYTES_PER_GRAIN = {"row_pred": 104.4, "col": 30.5, "row_corr": 133.2}
 
 
 def algorithmic_bytes(nx: int, ny: int, px: int, py: int, nl: int = 1, fp: int = 4, runs: int = 1,
@@ -72,10 +72,11 @@ def algorithmic_bytes(nx: int, ny: int, px: int, py: int, nl: int = 1, fp: int =
     tensor comes from another run of the same geometry share its buffer).
 
     row predictor: H^ rows in + M^ rows out (2 * 3 ny (px/2+1) complex), per grain
-      m, pa, pb (3 x 16 B), exchange CSR (4 B index + 4 x (4 B nbr + 4 B coef)),
-      writes m*, d (2 x 16 B)                     -> 116 B/grain
-    row corrector: same spectra, per grain m, m*, d, pa, pb (5 x 16 B),
-      CSR 36 B, writes m (16 B)                    -> 132 B/grain
+      m, pa (2 x 16 B), writes m*, d (2 x 16 B)   -> 64 B/grain
+    row corrector: same spectra, per grain m, m*, d, pa (4 x 16 B), writes
+      m (16 B)                                     -> 80 B/grain
+      (the exchange and the damping and Ms records of this medium are the same
+      at every grain, so one of each is read)
     column: M^ columns in + H^ out (2 * 3 ny (px/2+1) complex) per run, plus
       the tensor: one layer, the symmetric tensor's six components at every
       k_y of the (px/2+1) columns (the register column kernel's layout:
@@ -85,8 +86,8 @@ def algorithmic_bytes(nx: int, ny: int, px: int, py: int, nl: int = 1, fp: int =
     c = 2 * fp
     spec = 3 * nl * ny * (px // 2 + 1) * c
     n = nx * ny * nl
-    row_pred = 2 * spec + n * (3 * 16 + 36 + 2 * 16)
-    row_corr = 2 * spec + n * (5 * 16 + 36 + 16)
+    row_pred = 2 * spec + n * (2 * 16 + 2 * 16)
+    row_corr = 2 * spec + n * (4 * 16 + 16)
     tensor = ((px // 2 + 1) * 6 * py * fp if nl == 1 else (px // 2 + 1) * nl * nl * 9 * (py // 2 + 1) * fp)
     col = runs * 2 * spec + tensors * tensor
     return {"row_pred": runs * row_pred, "col": col, "row_corr": runs * row_corr}
@@ -697,7 +698,7 @@ def main():
                      "traffic": (NCU_TRAFFIC_BYTES_PER_GRAIN[dom] * nb * n
                                  if dom in NCU_TRAFFIC_BYTES_PER_GRAIN else None),
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per launch, 32 x 65,536 "
-                                       "grains, row shape 1, register column kernel 128 x 4, 1 column per task",
+                                       "grains, row shape 3, register column kernel in turn 128 x 3, 1 column per task",
                      "per_kernel_ms": per_kernel, "launches_per_heun_step": launches_per_heun,
                      "per_kernel_frac": {k: ab[k] / (v * 1e-3) / 1e9 / peak for k, v in per_kernel.items()},
                      "occupancy_blocks_per_sm": {"row": B["occupancy"][0], "col": B["occupancy"][1]},
