@@ -469,9 +469,17 @@ MRM_D bool creg_task_ok(const RunDev<float>& rd, int k0, int nc, int group, int 
 // us per Heun step, with 168 registers and two blocks per SM (80 registers
 // spill those loads).  On a batch by the shared-memory pipe (78 % of its
 // wavefronts): see below.
+//
+// Whether a task has work (its run is active and due) is thread 0's verdict,
+// taken when it issues the tiles, in a word of its own per slot that is read
+// only behind landed() of that task.  Everything read earlier, the choice of
+// the loop among it, is constant while the kernel runs, so every thread of the
+// block takes the same path and meets the same barriers: a task without work
+// meets one, in landed().
 struct CregTasks {
   alignas(16) unsigned char hdr[3][kRunHdrBytes];  // run headers of three consecutive tasks
-  int2 cols[3];                                    // their first column and columns (0: no work)
+  int2 cols[3];                                    // their first column and columns
+  int work[3];                                     // their tiles are on the way (thread 0's verdict)
   uint64_t bar;
 };
 
@@ -502,10 +510,8 @@ struct CregLoop {
     const bool live = h.active && h.demag && ((flags & kFlagForce) || step_due(h, step + istep));
     const bool ok = task_ok(slot);
     if (live && !ok) atomicOr(err, kErrShape);
-    if (!(live && ok)) {
-      ct->cols[slot].y = 0;
-      return;
-    }
+    ct->work[slot] = live && ok;
+    if (!(live && ok)) return;
     const int lgct = h.lgct, T = 1 << lgct, ph = (h.px >> 1) + 1, ntile = (ph + T - 1) >> lgct;
     const int ntl = (kc.y + T - 1) >> lgct, plane = (h.nys << lgct) * ntl;
     const Cx<float>* src = h.specx + (((size_t)(kc.x >> lgct) * h.nys) << lgct);
@@ -514,6 +520,8 @@ struct CregLoop {
       bulk_copy(&ct->bar, stg + q * plane, src + q * pstride, (uint32_t)(plane * sizeof(Cx<float>)));
   }
   int group, nl;    // the compiled shape
+  // (from the lengths and the table entry alone: the same for every thread at
+  // any time once the header has landed)
   MRM_D bool task_ok(int slot) const {
     const int2 kc = ct->cols[slot];
     return creg_task_ok(rd(slot), kc.x, kc.y, group, nl, tw_cap, stage_cap);
@@ -568,9 +576,8 @@ MRM_D bool creg_run(CregLoop& c, const float4* tw, float4* xb) {
       c.begin();
       if (!c.landed()) return false;
       const int2 kc = c.ct->cols[c.r];
-      if (kc.y == 0) {  // no work: the staging area was not written
-        __syncthreads();
-        c.issue_next();
+      if (!c.ct->work[c.r]) {
+        c.issue_next();  // (no tile of this task was copied, and every thread is past the last one's)
       } else {
         creg_body<LGN, G, NL, AHEAD, HALF>(rd, kc.x, kc.y, tens, tw, c.stg, xb, [&]() { c.issue_next(); });
       }
