@@ -2081,7 +2081,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) col_kernel(const RunDev<R>* __res
   pdl_launch_dependents();
   const Task tk = tasks[blockIdx.x];
   const RunDev<R>& rd = runs[tk.x];
-  if (!rd.active || !rd.demag) return;
+  if (!rd.active || !rd.demag) {
+    // (the wait also where there is no work: this launch covers only the
+    // in-place kernel's runs, and with all of them parked it would end before
+    // the row kernel that the next launch takes it to stand for)
+    pdl_wait();
+    return;
+  }
   const int k0 = tk.y, nc = tk.z;
   const int nl = rd.nl, py = rd.py, lgpy = rd.lgpy, lgct = rd.lgct;
   const int ph = (rd.px >> 1) + 1, pyhs = rd.pyhs;

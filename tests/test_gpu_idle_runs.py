@@ -102,3 +102,27 @@ def test_one_layer_budgets(gpulib, shape, rows):
     for i, (r, m, k) in enumerate(zip(runs, meds, ends)):
         _same(r, m, _alone(m, 70 + i, k if i % 2 == 0 else min(steps + 5, k + 25), shape))
     b.close()
+
+
+@pytest.mark.parametrize("ny", [128, 512])
+def test_parked_in_place_runs_beside_others(gpulib, ny):
+    """The in-place column kernel's launch covers only its own runs (here a
+    32-point one); with those parked, the launches behind it still follow the
+    row kernel of the runs that step: one with demag in the register column
+    kernel, one without demag."""
+    small, big = media.mh_medium(40, ny=16, seed=90, temperature=300.0), media.mh_medium(256, ny=ny, seed=91, temperature=300.0)
+    bare = media.mh_medium(1024, ny=512, seed=92, temperature=300.0)
+    b = Batch(FP32)
+    r0 = b.add(small, dt=DT, steps=40, thermal_seed=1)
+    r1 = b.add(big, dt=DT, steps=40, thermal_seed=2)
+    r2 = b.add(bare, dt=DT, steps=40, thermal_seed=3, demag=False)
+    r0.set_run(DT, 40, active=False)
+    b.step(40)
+    b.stats([r1, r2])
+    _same(r0, small, _alone(small, 1, 0))
+    _same(r1, big, _alone(big, 2, 40))
+    g = GpuSim(bare, precision=FP32, thermal_seed=3, demag=False)
+    g.step(40, DT)
+    _same(r2, bare, [g.get_state(0)])
+    g.close()
+    b.close()
