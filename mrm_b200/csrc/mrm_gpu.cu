@@ -420,11 +420,11 @@ int rows_per_task(const mrm_gpu* r, int rpb) { return r->wnx ? 1 : std::max(1, s
 // single runs whose blocks of six components crowd out the next kernel's early
 // start: 437 x 48 x 2 grains 54 us per step against 47 with the in-place kernel,
 // 500 x 75 x 2 60 against 54; 1024 x 256 x 2 190 against 235), with a symmetric
-// tensor: that kernel
-// keeps six components per layer pair (tensor.cuh pack_tensor_creg_kernel).
-// The SUL and head image terms make N_xz and N_zx differ; such a tensor keeps
-// its nine components and the in-place column kernel, which also takes the
-// other lengths and layer counts.
+// tensor (to kTensAsym of its largest value): that kernel keeps six components
+// per layer pair (tensor.cuh pack_tensor_creg_kernel).  The SUL and head image
+// terms make N_xz and N_zx differ; such a tensor keeps its nine components and
+// the in-place column kernel, which also takes the other lengths and layer counts.
+constexpr double kTensAsym = 0x1p-40;
 bool creg_shape(const mrm_gpu* r) {
   return r->g.precision == MRM_FP32 && r->nl <= 2 && r->lgpy >= (r->nl == 1 ? kCregMinLg : kCregMinLg2) &&
          r->lgpy <= kCregMaxLg && !r->fft_big;
@@ -1921,8 +1921,10 @@ int tensor_spectrum(mrm_gpu* r, const TensorScratch& w) {
     pack_tensor_creg_kernel<<<(unsigned)((total + 255) / 256), 256, 0, e->st>>>(
         d_spec, static_cast<float*>(r->tens), npair, r->lgpy, ph, d_mx);
     CK(read_maxima());
-    // symmetric to the rounding of the FP32 store (4 ulp of the largest value)
-    r->tens_sym = packed = !(mx[2] > 2.4e-7 * mx[1]);
+    // symmetric to the rounding of the FP64 transforms (a tensor without images
+    // is so exactly): a small N_xz - N_zx is not rounding of the FP32 store, whose
+    // error follows each component's own size
+    r->tens_sym = packed = !(mx[2] > kTensAsym * mx[1]);
   }
   if (!packed) {
     CK(cudaMemsetAsync(d_mx, 0, 3 * sizeof(unsigned long long), e->st));

@@ -95,3 +95,27 @@ def test_grain_records(oracle, gpulib, vary):
         assert np.abs(gpu.get_state(0) - orc.get_state(0)).max() < steps * 8 * 2.0**-24, row
         assert np.allclose(sg["mave"], so["mave"], rtol=0, atol=steps * 8 * 2.0**-24)
         gpu.close()
+
+
+def test_small_asymmetric_part(gpulib):
+    """Two layers with 512-point columns and a tensor of N_zz on the diagonal
+    with a small N_xz = -N_zx: moments along x see N_zx alone, so its sign shows
+    in H_z at full precision however small it is."""
+    med = _medium(8, 256, 2, 1)
+    gpu = GpuSim(med, precision=FP32)
+    px, py = gpu.fft_grid()
+    T = np.zeros((2, 2, 9, py, px))
+    T[:, :, 8, 0, 0] = 1.0 / (px * py)
+    # |N_xz - N_zx| is 1.2e-7 of the largest value in the spectrum
+    e = 3e-8 / (px * py)
+    T[:, :, 2, 0, 1], T[:, :, 2, 0, -1] = e, -e
+    T[:, :, 6] = -T[:, :, 2]
+    gpu.upload_tensor(T)
+    rng = np.random.default_rng(6)
+    ms = [np.outer(rng.choice([-1.0, 1.0], lay.N), [1.0, 0.0, 0.0]) for lay in med.layers]
+    want = _convolve(T, med, ms)
+    for l, m in enumerate(ms):
+        gpu.set_state(l, m)
+    for l in range(2):
+        assert rel_l2(gpu.eval_field(0.0, l)[:, 2], want[l][:, 2]) < DEMAG_TOL
+    gpu.close()
