@@ -430,16 +430,18 @@ bool creg_shape(const mrm_gpu* r) {
          r->lgpy <= kCregMaxLg && !r->fft_big;
 }
 bool creg_run(const mrm_gpu* r) { return creg_shape(r) && r->tens_sym; }
-// shape of the register column kernel: the column shape index, with the group
-// size of shape 1 (a single run's, registers before resident blocks) by the
-// longest columns
-int creg_v(const Engine* e) {
+// shape of the register column kernel for the runs of nl layers: the column
+// shape index, with the group size of shape 1 (a single run's, registers before
+// resident blocks) by their longest columns.  (Runs of one and of two layers
+// are launches of their own, so the long columns of a two-layer run do not
+// take the one-layer runs' groups from them.)
+int creg_v(const Engine* e, int nl) {
   const int v = std::min(std::max(e->colv, 0), kCregVariants - 1);
   bool fits = true, shorter = true;
   for (auto* r : e->runs) {
-    if (!creg_run(r)) continue;
-    fits = fits && creg_pairs(r->lgpy, kCreg[v].group[r->nl - 1]) >= 1;
-    shorter = shorter && creg_pairs(r->lgpy, kCreg[kCregShort].group[r->nl - 1]) >= 1;
+    if (!creg_run(r) || r->nl != nl) continue;
+    fits = fits && creg_pairs(r->lgpy, kCreg[v].group[nl - 1]) >= 1;
+    shorter = shorter && creg_pairs(r->lgpy, kCreg[kCregShort].group[nl - 1]) >= 1;
   }
   return v == 1 ? (shorter ? kCregShort : fits ? 1 : kCregLong) : fits ? v : 0;
 }
@@ -752,7 +754,7 @@ int plan_smem(Engine* e) {
   int need[kSlots] = {0, 0, 0, 0, 0, 0}, least[kSlots] = {0, 0, 0, 0, 0, 0};
   size_t scol = 16;
   int tw_cap[2] = {0, 0}, stage_bytes[2] = {0, 0};
-  const int cv = creg_v(e);
+  const int cv[2] = {creg_v(e, 1), creg_v(e, 2)};
   const RowPackCap pack = row_pack_cap<R>(e, rv.rpb);
   for (auto* r : e->runs) {
     if (r->lgpx > rv.lgmax)
@@ -768,7 +770,7 @@ int plan_smem(Engine* e) {
       if (creg_run(r)) {
         int &tw = tw_cap[r->nl - 1], &sb = stage_bytes[r->nl - 1];
         tw = std::max(tw, col_tw_count(r->lgpy));
-        sb = std::max(sb, creg_stage_of(cv, r));
+        sb = std::max(sb, creg_stage_of(cv[r->nl - 1], r));
       } else scol = std::max(scol, col_smem_of<R>(r, cols_per_task(e, r), col_variant<R>(e->colv).minb));
     }
   }
@@ -786,7 +788,7 @@ int plan_smem(Engine* e) {
   if (scol + 64 > kMaxSmem) return set_err(errp, MRM_ERR_UNSUPPORTED, "column shape exceeds shared memory");
   e->smem_col = scol;
   for (int i = 0; i < 2; ++i) {
-    const size_t screg = tw_cap[i] ? creg_smem_of(cv, i + 1, tw_cap[i], stage_bytes[i]) : 16;
+    const size_t screg = tw_cap[i] ? creg_smem_of(cv[i], i + 1, tw_cap[i], stage_bytes[i]) : 16;
     if (screg + kCregStatic > kMaxSmem) return set_err(errp, MRM_ERR_UNSUPPORTED, "column shape exceeds shared memory");
     e->smem_creg[i] = screg;
     e->creg_tw_cap[i] = tw_cap[i];
@@ -818,10 +820,10 @@ int plan_smem(Engine* e) {
   for (int i = 0; i < 2; ++i) {
     e->creg_blocks[i] = 0;
     if (sizeof(R) != sizeof(float) || !e->creg_tw_cap[i]) continue;
-    CK(creg_allow_smem(cv, i + 1, e->smem_creg[i]));
+    CK(creg_allow_smem(cv[i], i + 1, e->smem_creg[i]));
     // persistent blocks: as many as stay resident
     int per_sm = 0, sms = 0;
-    CK(creg_occupancy(cv, i + 1, e->smem_creg[i], &per_sm));
+    CK(creg_occupancy(cv[i], i + 1, e->smem_creg[i], &per_sm));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
     e->creg_blocks[i] = std::max(1, per_sm) * sms;
   }
@@ -834,7 +836,7 @@ int build_tables(Engine* e) {
   const RowVariant rv = row_variant<R>(e->rowv);
   const RowPackCap pack = row_pack_cap<R>(e, rv.rpb);
   std::vector<Task> rt, ct, ct2[2], stt;
-  const int cv = creg_v(e);
+  const int cv[2] = {creg_v(e, 1), creg_v(e, 2)};
   for (size_t i = 0; i < e->runs.size(); ++i) {
     mrm_gpu* r = e->runs[i];
     r->slot = (int)i;
@@ -851,7 +853,7 @@ int build_tables(Engine* e) {
       const int ph = r->px / 2 + 1;
       if (creg_run(r)) {
         // a task is what a block of the register column kernel holds
-        const int cpt = 2 * creg_pairs(r->lgpy, kCreg[cv].group[r->nl - 1]);
+        const int cpt = 2 * creg_pairs(r->lgpy, kCreg[cv[r->nl - 1]].group[r->nl - 1]);
         r->lgct = ilog2(col_tile(cpt));
         for (int k = 0; k < ph; k += cpt) ct2[r->nl - 1].push_back(make_int4((int)i, k, std::min(cpt, ph - k), 0));
       } else {
@@ -979,7 +981,7 @@ cudaError_t launch_col_e(Engine* e, int istep, int flags, bool pdl = true) {
     ColLaunch a{e->st, e->d_runs, e->d_ctasks2[q], e->d_tw, e->d_err, e->nct2[q], e->smem_creg[q], pdl};
     a.blocks = e->creg_blocks[q];
     a.tw_cap = e->creg_tw_cap[q];
-    const cudaError_t ce = launch_creg(creg_v(e), q + 1, a, istep, flags);
+    const cudaError_t ce = launch_creg(creg_v(e, q + 1), q + 1, a, istep, flags);
     if (ce != cudaSuccess) return ce;
   }
   return cudaSuccess;
@@ -3582,7 +3584,7 @@ static int occ_t(Engine* e, int* out2) {
     CK(row_occupancy<R>(e->rowv, kPred, e->smem_row[1], &a));
     // the column kernel of most of the batch's column tasks
     const int q = e->nct2[1] > e->nct2[0] ? 1 : 0;
-    if (e->nct2[q] > e->nct) CK(creg_occupancy(creg_v(e), q + 1, e->smem_creg[q], &b));
+    if (e->nct2[q] > e->nct) CK(creg_occupancy(creg_v(e, q + 1), q + 1, e->smem_creg[q], &b));
     else CK(col_occupancy<R>(e->colv, e->smem_col, &b));
   }
   out2[0] = a;
