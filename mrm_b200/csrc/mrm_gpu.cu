@@ -1076,9 +1076,11 @@ void default_shapes(Engine* e) {
 }
 
 // signature of a batch for the tuner's cache: precision, largest grid, layers,
-// order of magnitude of the grain count
+// order of magnitude of the grain count, and the longest columns in each of the
+// column launches (in-place, register of one and of two layers; 0: none), since
+// the column shape and the columns per task were timed for those kernels
 std::string shape_key(const Engine* e) {
-  int lgx = 0, lgy = 0, nl = 0;
+  int lgx = 0, lgy = 0, nl = 0, col[3] = {0, 0, 0};
   long long grains = 0;
   for (auto* r : e->runs) {
     if (!r->active) continue;
@@ -1086,9 +1088,14 @@ std::string shape_key(const Engine* e) {
     lgy = std::max(lgy, r->lgpy);
     nl = std::max(nl, r->nl);
     grains += (long long)r->g.nx * r->g.ny * r->nl;
+    if (r->demag && r->tensor_ready) {
+      int& c = col[creg_run(r) ? r->nl : 0];
+      c = std::max(c, r->lgpy);
+    }
   }
-  char buf[96];
-  std::snprintf(buf, sizeof buf, "%d/%d/%d/%d/%d/%d", e->dev, e->prec, lgx, lgy, nl, grains > 0 ? ilog2((int)std::min<long long>(grains, 1LL << 30)) : 0);
+  char buf[128];
+  std::snprintf(buf, sizeof buf, "%d/%d/%d/%d/%d/%d/%d/%d/%d", e->dev, e->prec, lgx, lgy, nl,
+                grains > 0 ? ilog2((int)std::min<long long>(grains, 1LL << 30)) : 0, col[0], col[1], col[2]);
   return buf;
 }
 
@@ -1105,18 +1112,22 @@ std::map<std::string, Shape>& tune_cache() {
 // batch itself (one Heun step's chained launches, as the captured steps run
 // them) and keeps the fastest.  The
 // kernels run on the real state, which is saved before and restored after
-// (m and the stored field per layer; the spectra are re-established).
+// (m and the stored field per layer; the spectra are re-established).  A batch
+// with the signature of an earlier one takes that one's shapes (*cached) unless
+// `fresh`.
 template <typename R>
-int autotune(Engine* e) {
+int autotune(Engine* e, bool fresh, bool* cached) {
   std::string* errp = &e->err;
   const std::string key = shape_key(e);
-  {
+  *cached = false;
+  if (!fresh) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = tune_cache().find(key);
     if (it != tune_cache().end()) {
       e->rowv = it->second.rowv;
       e->colv = it->second.colv;
       e->cpt = it->second.cpt;
+      *cached = true;
       return MRM_OK;
     }
   }
@@ -1230,6 +1241,7 @@ int ensure_ready(Engine* e) {
   std::string* errp = &e->err;
   CK(cudaSetDevice(e->dev));
   if (e->tables_dirty) {
+    bool cached = false;
     if (e->shape_forced) {
       e->rowv = e->force_rowv;
       e->colv = e->force_colv;
@@ -1239,13 +1251,19 @@ int ensure_ready(Engine* e) {
       bool ready = true;
       for (auto* r : e->runs)
         if (r->active && r->demag && !r->tensor_ready) ready = false;
-      int rc = ready ? autotune<R>(e) : MRM_OK;
+      int rc = ready ? autotune<R>(e, false, &cached) : MRM_OK;
       if (!ready) default_shapes<R>(e);
       if (rc) return rc;
     } else {
       default_shapes<R>(e);
     }
     int rc = build_tables<R>(e);
+    if (rc == MRM_ERR_UNSUPPORTED && cached) {
+      // (shapes tuned on another batch that this one's shared memory does not take)
+      e->err.clear();
+      rc = autotune<R>(e, true, &cached);
+      if (!rc) rc = build_tables<R>(e);
+    }
     if (rc) return rc;
   }
   if (e->desc_dirty) {

@@ -30,3 +30,50 @@ def test_long_two_layer_columns_leave_the_one_layer_runs_alone(gpulib):
             g.close()
         b.close()
     assert occ[0] == occ[1] > 2, occ
+
+
+def _images(med):
+    """A soft underlayer: its image terms make the tensor asymmetric, which the
+    in-place column kernel takes."""
+    med.sul_mu, med.space_to_sul = 50.0, 2e-7
+    return med
+
+
+def _step_all(meds, n=8):
+    b = Batch(FP32)
+    same, runs = {}, []
+    for i, m in enumerate(meds):
+        key = (m.nx, m.ny, m.n_lay)
+        runs.append(b.add(m, dt=1e-13, steps=n, thermal_seed=7, tensor_from=same.get(key)))
+        same.setdefault(key, runs[-1])
+    b.step(n)
+    b.stats(runs)
+    shape, out = runs[0].get_shape(), [[r.get_state(l) for l in range(m.n_lay)] for r, m in zip(runs, meds)]
+    b.close()
+    return shape, out
+
+
+def test_tuned_shapes_follow_the_column_kernel(gpulib):
+    """One column per task is all a batch of the register kernel has to time (it
+    does not use the number); a batch of the in-place kernel with the same sizes
+    times its own, and one column per task is never the fastest there (81 or 68 us
+    a launch against 62 with two)."""
+    med = media.mh_medium(256, seed=3)
+    assert _step_all([med] * 16)[0][2] == 1
+    assert _step_all([_images(media.mh_medium(256, seed=3))] * 16)[0][2] > 1
+
+
+def test_tuned_shapes_that_do_not_fit_are_tuned_again(gpulib):
+    """Short in-place columns are fastest at many columns per task; the same
+    batch with its long two-layer run on the in-place kernel as well has no
+    shared memory for that many."""
+    short = _images(media.mh_medium(128, seed=3))
+    sym = media.two_layer_medium(24, 512, seed=9, temperature=0.0)
+    asym = _images(media.two_layer_medium(24, 512, seed=9, temperature=0.0))
+    _step_all([short] * 32 + [sym])
+    _, out = _step_all([short] * 32 + [asym])
+    g = GpuSim(asym, precision=FP32, thermal_seed=7)
+    g.step(8, 1e-13)
+    for l in range(2):
+        assert np.array_equal(out[-1][l], g.get_state(l)), l
+    g.close()
