@@ -556,7 +556,7 @@ struct CregLoop {
     if (!first) return;
     first = false;
     pdl_wait();
-    if (threadIdx.x == 0) issue(r, i, run_step(runs[tasks[i].x]));
+    if (threadIdx.x == 0) issue(r, i, *reinterpret_cast<const volatile long long*>(&runs[tasks[i].x].step));
   }
   MRM_D void advance() {
     i += (int)gridDim.x;
@@ -894,7 +894,7 @@ __global__ void __launch_bounds__(G, MINB)
     i += gridDim.x;
     if (i < ntasks) tk = tasks[i];
     const int lgpy = rd.lgpy, T = 1 << rd.lgct, ph = (rd.px >> 1) + 1;
-    const bool work = rd.active && rd.demag && ((flags & kFlagForce) || step_due(rd, run_step(rd) + istep));
+    const bool work = rd.active && rd.demag && ((flags & kFlagForce) || step_due(rd, rd.step + istep));
     const bool ok = lgpy >= kCregMinLg && lgpy <= kCregMaxLg && (8 * G >> lgpy) >= 1 && rd.nl == 1 && nc >= 1 &&
                     k0 >= 0 && (k0 & 1) == 0 && k0 + nc <= ph && nc <= 2 * creg_pairs(lgpy, G) && T >= 2 &&
                     col_tw_count(lgpy) <= tw_room;

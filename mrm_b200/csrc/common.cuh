@@ -226,14 +226,6 @@ template <typename R>
 MRM_HD bool step_due(const RunDev<R>& rd, long long step) {
   return step >= rd.step_begin && step < rd.step_end;
 }
-// The run's step counter, to be read behind the dependency wait: advance_kernel
-// writes it.  Other fields of the descriptor, which no kernel writes, are read
-// before that wait as well, so a plain load could be served from a line of the
-// first-level cache that is older than the counter.
-template <typename R>
-MRM_D long long run_step(const RunDev<R>& rd) {
-  return *reinterpret_cast<const volatile long long*>(&rd.step);
-}
 
 // row task: (run, layer, first row, number of rows); column task: (run, first column, ncols, 0)
 using Task = int4;
