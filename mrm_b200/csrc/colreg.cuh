@@ -894,6 +894,7 @@ __global__ void __launch_bounds__(G, MINB)
     i += gridDim.x;
     if (i < ntasks) tk = tasks[i];
     const int lgpy = rd.lgpy, T = 1 << rd.lgct, ph = (rd.px >> 1) + 1;
+    // (the step counter does not change while this kernel is resident: advance_kernel)
     const bool work = rd.active && rd.demag && ((flags & kFlagForce) || step_due(rd, rd.step + istep));
     const bool ok = lgpy >= kCregMinLg && lgpy <= kCregMaxLg && (8 * G >> lgpy) >= 1 && rd.nl == 1 && nc >= 1 &&
                     k0 >= 0 && (k0 & 1) == 0 && k0 + nc <= ph && nc <= 2 * creg_pairs(lgpy, G) && T >= 2 &&

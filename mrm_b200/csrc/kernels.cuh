@@ -2137,7 +2137,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) col_kernel(const RunDev<R>* __res
     mbar_arrive(&bars[0]);
   }
   pdl_wait();
-  const bool run_it = (flags & kFlagForce) || step_due(rd, rd.step + istep);
+  const bool run_it = (flags & kFlagForce) || step_due(rd, rd.step + istep);  // (advance_kernel)
   const bool ok = mbar_wait(&bars[0], 0);
   if (__syncthreads_or(!ok)) {
     if (threadIdx.x == 0) atomicOr(err, kErrBarrierTimeout);
@@ -2291,9 +2291,12 @@ __global__ void __launch_bounds__(256) commit_kernel(const RunDev<R>* __restrict
 }
 
 // Advances every active run's step counter after a captured chunk of k steps.
+// It does not let its dependents start early: the kernels behind it read other
+// fields of a descriptor ahead of their dependency wait, and the line of the
+// first-level cache that this brings in must hold the new counter (the column
+// kernels read it with plain loads).
 template <typename R>
 __global__ void advance_kernel(RunDev<R>* runs, int nruns, int k) {
-  pdl_launch_dependents();
   pdl_wait();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nruns) return;
