@@ -478,6 +478,20 @@ constexpr size_t kCregStatic = 768;
 constexpr size_t kSmemPerSM = 228 * 1024;
 constexpr size_t kSmemReserved = 1024;  // per block
 
+// Shared memory that a row launch of `tasks` blocks asks for beyond what it uses,
+// beside the in-place column kernel of FP32 runs: just over a share of one more
+// block per SM than an even spread needs (at least two), so that no more fit.
+// Row blocks start while the column kernel's are still resident, wherever there
+// is room; with the 20 to 40 KB that they use, three or four go to one SM while
+// others have none, and the launch waits for those.  Two-layer runs, us per Heun
+// step without / with: 700 x 60 (120 blocks) 82.7 / 71.8, 537 x 120 (240) 105.2 /
+// 98.0, 600 x 200 (400) 152.9 / 139.0; 437 x 48 (96) 48.4 / 46.4, and 48.4 with
+// room for one.  Four per SM is what the registers hold anyway.
+size_t row_spread_smem(int tasks, int sms, size_t static_bytes) {
+  const int per_sm = std::max(2, (tasks + sms - 1) / sms);
+  return per_sm > 3 ? 0 : kSmemPerSM / (per_sm + 1) + 1024 - kSmemReserved - static_bytes;
+}
+
 // staging bytes a run needs at a stage (largest over its layers)
 template <typename R>
 int run_stage_bytes(const mrm_gpu* r, int stage, int rows) {
@@ -793,6 +807,12 @@ int plan_smem(Engine* e) {
     e->smem_creg[i] = screg;
     e->creg_tw_cap[i] = tw_cap[i];
   }
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
+  const bool spread = sizeof(R) == sizeof(float) && e->nct && !e->nct2[0] && !e->nct2[1];
+  if (spread)
+    for (int q = 0; q < kSlots; ++q)
+      e->smem_row[q] = std::max(e->smem_row[q], row_spread_smem(e->nrt, sms, row_static_bytes(q)));
   CK(row_allow_smem<R>(e->rowv, e->smem_row));
   // the reductions launches (kPred of the single-stage integrator, kCorr):
   // row shape 0, one row per task
@@ -812,6 +832,7 @@ int plan_smem(Engine* e) {
     for (int i = 0; i < 2; ++i) {
       e->cap_stats[i] = (int)(std::min<long long>(n0[i], std::max(0LL, std::min(per_block, hard))) & ~15LL);
       e->smem_stats[i] = f0 + (size_t)e->cap_stats[i];
+      if (spread) e->smem_stats[i] = std::max(e->smem_stats[i], row_spread_smem(e->nst, sms, row_static_bytes(3)));
     }
     size_t lim[kSlots] = {0, 0, 0, e->smem_stats[1], 0, e->smem_stats[0]};
     CK(row_allow_smem<R>(0, lim));
@@ -822,9 +843,8 @@ int plan_smem(Engine* e) {
     if (sizeof(R) != sizeof(float) || !e->creg_tw_cap[i]) continue;
     CK(creg_allow_smem(cv[i], i + 1, e->smem_creg[i]));
     // persistent blocks: as many as stay resident
-    int per_sm = 0, sms = 0;
+    int per_sm = 0;
     CK(creg_occupancy(cv[i], i + 1, e->smem_creg[i], &per_sm));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
     e->creg_blocks[i] = std::max(1, per_sm) * sms;
   }
   return MRM_OK;

@@ -77,3 +77,17 @@ def test_tuned_shapes_that_do_not_fit_are_tuned_again(gpulib):
     for l in range(2):
         assert np.array_equal(out[-1][l], g.get_state(l)), l
     g.close()
+
+
+@pytest.mark.parametrize("layers,ny,most", [(2, 48, 2), (2, 100, 2), (1, 400, 3), (1, 512, 4)])
+def test_row_blocks_spread_over_the_sms(gpulib, layers, ny, most):
+    """Runs of the in-place column kernel: no more row blocks fit an SM than an
+    even spread of the launch needs, at least two."""
+    med = media.two_layer_medium(437, ny, seed=4) if layers == 2 else _images(media.mh_medium(437, ny=ny, seed=4))
+    b = Batch(FP32)
+    r = b.add(med, dt=1e-13, steps=10)
+    r.set_shape(0, 2, 2)
+    b.step(10)
+    b.stats([r])
+    assert b.occupancy()[0] == most
+    b.close()
