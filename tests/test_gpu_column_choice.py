@@ -91,3 +91,14 @@ def test_row_blocks_spread_over_the_sms(gpulib, layers, ny, most):
     b.stats([r])
     assert b.occupancy()[0] == most
     b.close()
+
+
+def test_row_blocks_of_a_small_run_keep_their_room(gpulib):
+    """65 column tasks leave more than half of the SMs to the row blocks."""
+    b = Batch(FP32)
+    r = b.add(_images(media.mh_medium(64, seed=4)), dt=1e-13, steps=10)
+    r.set_shape(0, 2, 1)
+    b.step(10)
+    b.stats([r])
+    assert b.occupancy()[0] == 4
+    b.close()
