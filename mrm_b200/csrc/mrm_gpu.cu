@@ -1078,17 +1078,24 @@ int establish_spectra(Engine* e) {
 // ---------------- shapes: default heuristic and autotuner ----------------
 template <typename R>
 void default_shapes(Engine* e) {
-  int maxnx = 1, maxlg = 1;
+  int maxnx = 1, maxlg = 1, sms = 148;
+  long long rows = 0;
   for (auto* r : e->runs) {
     maxnx = std::max(maxnx, fnx(r));
     maxlg = std::max(maxlg, r->lgpx);
+    if (r->active) rows += (long long)r->nl * fny(r);
   }
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev) != cudaSuccess) cudaGetLastError();
+  // (two rows to a 128-thread block need three rows per SM: one row to a 256-thread
+  // block and two to a 128-thread one, 128 x 128 grains, us per Heun step: one run
+  // 31.7 and 40.3, two 43.1 and 45.5, four 48.1 and 46.7, eight 64.5 and 53.7, 32
+  // runs 167 and 109)
   // rows per block so that a block holds about 256 grains
   const int want = std::max(1, 256 / maxnx);
   int best = 0;
   for (int v = 0; v < row_variant_count<R>(); ++v) {
     const RowVariant rv = row_variant<R>(v);
-    if (rv.lgmax < maxlg || rv.block != 256) continue;
+    if (rv.lgmax < maxlg || (rv.block != 256 && (rv.rpb == 1 || rows < 3LL * sms))) continue;
     const RowVariant bv = row_variant<R>(best);
     if (std::abs(rv.rpb - want) < std::abs(bv.rpb - want)) best = v;
   }

@@ -102,3 +102,22 @@ def test_row_blocks_of_a_small_run_keep_their_room(gpulib):
     b.stats([r])
     assert b.occupancy()[0] == 4
     b.close()
+
+
+@pytest.mark.parametrize("runs,row", [(1, 0), (8, 2)])
+def test_rows_per_block_without_the_tuner(gpulib, runs, row):
+    """Rows of 128 grains go two to a block where there are enough of them."""
+    med = media.mh_medium(128, seed=4, temperature=300.0)
+    b = Batch(FP32)
+    rs = []
+    for i in range(runs):
+        rs.append(b.add(med, dt=1e-13, steps=8, thermal_seed=3, tensor_from=rs[0] if rs else None))
+    rs[0].set_autotune(False)
+    b.step(8)
+    b.stats(rs)
+    assert rs[0].get_shape()[0] == row
+    g = GpuSim(med, precision=FP32, thermal_seed=3)
+    g.step(8, 1e-13)
+    assert np.array_equal(rs[-1].get_state(0), g.get_state(0))
+    g.close()
+    b.close()
