@@ -1080,10 +1080,12 @@ template <typename R>
 void default_shapes(Engine* e) {
   int maxnx = 1, maxlg = 1, sms = 148;
   long long rows = 0;
+  bool creg = false;
   for (auto* r : e->runs) {
     maxnx = std::max(maxnx, fnx(r));
     maxlg = std::max(maxlg, r->lgpx);
     if (r->active) rows += (long long)r->nl * fny(r);
+    creg = creg || (r->demag && creg_run(r));
   }
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev) != cudaSuccess) cudaGetLastError();
   // (two rows to a 128-thread block need three rows per SM: one row to a 256-thread
@@ -1100,7 +1102,11 @@ void default_shapes(Engine* e) {
     if (std::abs(rv.rpb - want) < std::abs(bv.rpb - want)) best = v;
   }
   e->rowv = best;
-  e->colv = 0;
+  // (the register column kernel's shape 1 is as fast as the others or faster in
+  // all but large runs and batches, where it costs 2 %: us per Heun step in shapes
+  // 0 / 1 / 2, 32 x 32 grains 29.6 / 23.4 / 29.3, 64 runs of it 48.6 / 33.2 / 44.3,
+  // 256 x 256 46.3 / 36.8 / 46.2, 512 x 512 70.9 / 72.7 / 72.1)
+  e->colv = creg ? 1 : 0;
   e->cpt = 0;
 }
 

@@ -121,3 +121,14 @@ def test_rows_per_block_without_the_tuner(gpulib, runs, row):
     assert np.array_equal(rs[-1].get_state(0), g.get_state(0))
     g.close()
     b.close()
+
+
+def test_column_shape_without_the_tuner(gpulib):
+    """Shape 1 of the register column kernel, shape 0 of the in-place one."""
+    for med, col in ((media.mh_medium(32, seed=4), 1), (_images(media.mh_medium(32, seed=4)), 0),
+                     (media.two_layer_medium(8, 500, seed=4), 1), (media.two_layer_medium(8, 20, seed=4), 0)):
+        g = GpuSim(med, precision=FP32)
+        g.set_autotune(False)
+        g.step(8, 1e-13)
+        assert g.get_shape()[1] == col
+        g.close()
