@@ -367,7 +367,8 @@ int mrm_gpu_off_field(mrm_gpu* h, double zoff, double dzobs, double head_mu, dou
  * (rows per block, threads, resident blocks; threads and resident blocks of
  * the column kernel) and cols_per_task > 0 fixes the spectral columns per
  * column task (rounded down to a power of two, at most 8: the width of the
- * column tiles the row kernel writes the M spectrum in); a negative shape returns to the automatic choice.  Results do
+ * column tiles the row kernel writes the M spectrum in); a negative shape returns to the automatic choice.  FP32 row
+ * shape 2 stands for shape 0 where the longest rows have a 2048-column FFT grid.  Results do
  * not depend on the shape.  Automatic: with autotuning on (the default), the
  * first step after the set of runs changes times every compiled shape on the
  * runs themselves (their state is restored) and keeps the fastest, cached per

@@ -18,7 +18,7 @@ struct RowVariant {
 };
 constexpr int kRowVariantsF32 = 5;
 constexpr RowVariant kRowF32[kRowVariantsF32] = {
-    {1, 256, 4, 12}, {1, 128, 8, 12}, {2, 128, 8, 11}, {4, 256, 4, 10}, {8, 256, 2, 8}};
+    {1, 256, 4, 12}, {1, 128, 8, 12}, {2, 128, 8, 10}, {4, 256, 4, 10}, {8, 256, 2, 8}};
 constexpr int kRowVariantsF64 = 3;
 constexpr RowVariant kRowF64[kRowVariantsF64] = {{1, 256, 2, 12}, {2, 256, 2, 11}, {8, 256, 1, 8}};
 template <typename R>

@@ -1281,6 +1281,12 @@ int ensure_ready(Engine* e) {
       e->rowv = e->force_rowv;
       e->colv = e->force_colv;
       e->cpt = e->force_cpt;
+      // (FP32 shape 2 is accepted for rows of up to 1024 columns; those beyond its
+      // compiled lengths run one to a block: compiled in, they cost its other
+      // lengths 1 to 3 %)
+      int lgx = 0;
+      for (auto* r : e->runs) lgx = std::max(lgx, r->lgpx);
+      if (sizeof(R) == sizeof(float) && e->rowv == 2 && lgx == row_variant<R>(2).lgmax + 1) e->rowv = 0;
     } else if (e->autotune) {
       // tuning needs every active run uploaded with its tensor
       bool ready = true;
