@@ -60,13 +60,13 @@ WORKLOAD = ("batched {b} x 65,536-grain M(H) ramp realisations, T=300 K, FP32, "
 # DRAM traffic per launch of each kernel in bytes per grain of the launch:
 # dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of the
 # headline batch (32 x 65,536 grains, row shape 3, the register column kernel
-# in turn {128 threads, 3 blocks/SM}, one column per task), divided by its
+# in turn {128 threads, 3 blocks/SM}, four columns per task), divided by its
 # grains; a kernel change calls for a new capture
 NCU_TRAFFIC_BYTES_PER_GRAIN = {"row_pred": 104.4, "col": 30.5, "row_corr": 133.2}
 
 
 def algorithmic_bytes(nx: int, ny: int, px: int, py: int, nl: int = 1, fp: int = 4, runs: int = 1,
-                      tensors: int = 1) -> dict:
+                      tensors: int = 1, uniform: bool = True) -> dict:
     """Bytes each kernel must move at minimum with this path's data layout, for
     `runs` runs of one geometry that read `tensors` tensor copies (runs whose
     tensor comes from another run of the same geometry share its buffer).
@@ -75,20 +75,28 @@ def algorithmic_bytes(nx: int, ny: int, px: int, py: int, nl: int = 1, fp: int =
       m, pa (2 x 16 B), writes m*, d (2 x 16 B)   -> 64 B/grain
     row corrector: same spectra, per grain m, m*, d, pa (4 x 16 B), writes
       m (16 B)                                     -> 80 B/grain
-      (the exchange and the damping and Ms records of this medium are the same
-      at every grain, so one of each is read)
+      (uniform: the exchange and the damping and Ms records are the same at
+      every grain, so one of each is read; otherwise 2 x 16 B a grain more)
     column: M^ columns in + H^ out (2 * 3 ny (px/2+1) complex) per run, plus
-      the tensor: one layer, the symmetric tensor's six components at every
-      k_y of the (px/2+1) columns (the register column kernel's layout:
-      6 py reals per column); more layers, nine components per layer pair at
-      0 <= k_y <= py/2
+      the tensor in the layout of the run's column kernel: the register ones
+      (FP32, no images, one layer with py = 64..1024 or two with 512 or 1024)
+      six components per layer pair at every k_y; the in-place one nine, in
+      FP32 at 0 <= k_y <= py/2, in FP64 complex at every k_y
     """
     c = 2 * fp
     spec = 3 * nl * ny * (px // 2 + 1) * c
     n = nx * ny * nl
-    row_pred = 2 * spec + n * (2 * 16 + 2 * 16)
-    row_corr = 2 * spec + n * (4 * 16 + 16)
-    tensor = ((px // 2 + 1) * 6 * py * fp if nl == 1 else (px // 2 + 1) * nl * nl * 9 * (py // 2 + 1) * fp)
+    rec = 4 * fp  # a grain's record
+    records = 0 if uniform else 2 * rec
+    row_pred = 2 * spec + n * (2 * rec + 2 * rec + records)
+    row_corr = 2 * spec + n * (4 * rec + rec + records)
+    if fp == 8:
+        reals = 9 * 2 * py
+    elif (nl == 1 and 64 <= py <= 1024) or (nl == 2 and py in (512, 1024)):
+        reals = 6 * py
+    else:
+        reals = 9 * (py // 2 + 1)
+    tensor = (px // 2 + 1) * nl * nl * reals * fp
     col = runs * 2 * spec + tensors * tensor
     return {"row_pred": runs * row_pred, "col": col, "row_corr": runs * row_corr}
 
@@ -698,7 +706,7 @@ def main():
                      "traffic": (NCU_TRAFFIC_BYTES_PER_GRAIN[dom] * nb * n
                                  if dom in NCU_TRAFFIC_BYTES_PER_GRAIN else None),
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per launch, 32 x 65,536 "
-                                       "grains, row shape 3, register column kernel in turn 128 x 3, 1 column per task",
+                                       "grains, row shape 3, register column kernel in turn 128 x 3, 4 columns per task",
                      "per_kernel_ms": per_kernel, "launches_per_heun_step": launches_per_heun,
                      "per_kernel_frac": {k: ab[k] / (v * 1e-3) / 1e9 / peak for k, v in per_kernel.items()},
                      "occupancy_blocks_per_sm": {"row": B["occupancy"][0], "col": B["occupancy"][1]},
