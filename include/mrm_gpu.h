@@ -372,8 +372,8 @@ int mrm_gpu_off_field(mrm_gpu* h, double zoff, double dzobs, double head_mu, dou
  * not depend on the shape.  Automatic: with autotuning on (the default), the
  * first step after the set of runs changes times every compiled shape on the
  * runs themselves (their state is restored) and keeps the fastest, cached per
- * grid size, layer count and grain-count magnitude; with it off, a size
- * heuristic.  mrm_gpu_get_shape: out3 = {row shape, column shape, columns per
+ * grid size, layer count, grain-count magnitude and the longest columns of each
+ * column kernel in use; with it off, a size heuristic.  mrm_gpu_get_shape: out3 = {row shape, column shape, columns per
  * task (0: default)} of the last step. */
 int mrm_gpu_set_shape(mrm_gpu* h, int row_shape, int col_shape, int cols_per_task);
 int mrm_gpu_set_autotune(mrm_gpu* h, int on);

@@ -464,9 +464,9 @@ MRM_D bool creg_task_ok(const RunDev<float>& rd, int k0, int nc, int group, int 
 // before the previous kernel has finished.  The twiddles are expanded again
 // only when the next task's column length differs.
 // Bound, in a single run, by the latency of one task's chain of stages (129
-// tasks on 148 SMs at 256 x 256): the tensor loaded ahead and the first
-// descriptor before the dependency wait took a 256 x 256 run from 48.0 to 38.2
-// us per Heun step, with 168 registers and two blocks per SM (80 registers
+// tasks on 148 SMs at 256 x 256): with the tensor loaded ahead and the first
+// descriptor before the dependency wait, at 168 registers and two blocks per SM,
+// a 256 x 256 run takes 38.2 us per Heun step, and 48.0 without (80 registers
 // spill those loads).  On a batch by the shared-memory pipe (78 % of its
 // wavefronts): see below.
 //
@@ -860,13 +860,13 @@ MRM_D void cser_column(const RunDev<float>& rd, int k0, int nc, const Cx<float>*
 
 // Persistent blocks: block b takes tasks b, b + B, b + 2B, ... (B blocks), its
 // next task's table entry loaded while the current one runs.
-// Measured on 32 runs of 256 x 256 grains, per launch: 94 us with one column
-// per thread group and 8-byte accesses (36 M warp instructions), 86 us with the
-// components side by side, 72 us in turn (22.7 M; 168 registers, 12 warps per
-// SM, so still latency: a third of its stalls are global loads, a fifth shared
-// ones).  Loading the next task's inputs ahead spilled (76 us); the tensor two
-// chunks ahead instead of one changed nothing.  Eight runs of 512 x 512: 103 ->
-// 87 us.
+// Measured on 32 runs of 256 x 256 grains, per launch: 72 us (22.7 M warp
+// instructions; 168 registers, 12 warps per SM, so bound by latency: a third of
+// its stalls are global loads, a fifth shared ones), 86 us with the components
+// side by side, 94 us with one column per thread group and 8-byte accesses
+// (36 M); eight runs of 512 x 512 87 us, and 103 in the last form.  Loading the
+// next task's inputs ahead spills (76 us); the tensor two chunks ahead instead
+// of one changes nothing.
 template <int G, int MINB>
 __global__ void __launch_bounds__(G, MINB)
     cser_kernel(const RunDev<float>* __restrict__ runs, const Task* __restrict__ tasks, int ntasks,

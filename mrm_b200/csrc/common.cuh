@@ -203,9 +203,11 @@ struct alignas(16) RunDev {
   // from grid column wi0, row wj0 of the full gnx x gny grid of the per-grain
   // arrays; frz: the run's first stats record of the frozen grains (-1: none)
   int gnx, gny, wi0, wj0, frz;
-  const R* tens;           // tensor spectrum: FP32 packed [px/2+1][nl*nl][9][pyhs] reals,
-                           // FP64 full [px/2+1][nl*nl][9][py] complex, each column in the
-                           // digit-reversed order of the column transform
+  const R* tens;           // tensor spectrum.  FP64: full [px/2+1][nl*nl][9][py] complex, each
+                           // column in the digit-reversed order of the column transform.  FP32,
+                           // in-place column kernel: packed [px/2+1][nl*nl][9][pyhs] reals; register
+                           // column kernels: [column pair][nl*nl][6][4][py/8][2][2] reals
+                           // (creg_tensor_reals in colreg.cuh)
   LayerDev<R> L[kMaxLayers];
 };
 

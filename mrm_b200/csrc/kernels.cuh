@@ -17,14 +17,13 @@
 // What bounds the row kernel: on a batch, instruction issue (55 % of the slots)
 // and the latency of its grain loads; in a single run, whose 256 rows leave two
 // blocks to an SM, the chain copy -> inverse transform -> grains -> forward
-// transform of one row (about 1.5 + 2.3 + 2.5 + 2.6 us at 256 x 256).  Measured
-// per launch on 32 runs of 256 x 256 grains (predictor / corrector):
-// 126 / 126 us with two FFT buffers per sequence, the stage's scalars computed
-// by every thread, the spectrum post-processing one value at a time and a grain
-// record loaded per grain; 107 / 108 us with one buffer (rows transformed in
-// place), shared scalars, post-processing in pairs, uniform records read once,
-// waits without polling and two rows to a 128-thread block.  The two-layer
-// write's 1024-point rows, four blocks to an SM instead of two: 93 -> 56 us.
+// transform of one row (about 1.5 + 2.3 + 2.5 + 2.6 us at 256 x 256).  Hence one
+// FFT buffer per sequence (rows transformed in place: four blocks of 1024-point
+// rows to an SM, 56 us a launch of a 1024 x 256 x 2 write, where two buffers
+// leave two and take 93), the stage's scalars computed once per block, the
+// spectrum post-processed in pairs, uniform records read once and waits without
+// polling: 102 / 105 us per launch (predictor / corrector) on 32 runs of
+// 256 x 256 grains, 126 / 126 without them.
 #pragma once
 #include "common.cuh"
 #include "fft.cuh"
@@ -393,9 +392,7 @@ static __device__ __noinline__ LlbStep llb_heun(bool corr, const double* mc, dou
   }
   // (one reciprocal for each divisor and one exponential for both functions of
   // x: an FP64 division or transcendental is a chain of dependent FMAs, and a
-  // run of one grain per thread waits for the sum of them.  256 x 256 LLB run,
-  // with the uniform-record masks kept out of these kernels as well: 81.8 -> 72.1
-  // us per Heun step)
+  // run of one grain per thread waits for the sum of them)
   double ht3[3];
   for (int a = 0; a < 3; ++a) ht3[a] = h[a] + lam * mag * m[a];
   const double mh = sqrt(ht3[0] * ht3[0] + ht3[1] * ht3[1] + ht3[2] * ht3[2]);
@@ -1899,9 +1896,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) row_kernel(const RunDev<R>* __res
 // The tensor of a task's columns is staged in shared memory, by a bulk copy ahead
 // of the dependency wait, up to 48 KB in FP32 and 80 KB in FP64 (one 512-point
 // column's nine complex components, 74 KB): the product then waits for no
-// global load.  (256 x 256 FP64 run, with the FP64 tensor in the order of the
-// transform's positions so that a warp reads consecutive values: 63.1 -> 49.5 us
-// per step; 64 x 64: 27.7 -> 26.7.)
+// global load.  The FP64 tensor is in the order of the transform's positions, so
+// a warp reads consecutive values.  (256 x 256 FP64 run 49.5 us per step, and 63.1
+// read from global memory in k_y order.)
 template <typename R>
 MRM_HD int tens_slice_reals(int nc, int npair, int py, int pyhs) {
   return nc * npair * 9 * (sizeof(R) == sizeof(float) ? pyhs : 2 * py);

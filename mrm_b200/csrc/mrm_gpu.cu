@@ -248,8 +248,8 @@ void dfree(void*& p) {
 // One device allocation for the temporaries of a call, each piece on a
 // 256-byte boundary, given back when the object goes out of scope.  Not
 // zero-filled: every piece is written before it is read, in stream order.
-// (A call that took each piece with dmalloc paid a cudaMalloc, a cleared copy
-// of the piece, a synchronisation and a cudaFree for every one of them.)
+// (dmalloc would cost a cudaMalloc, a clear, a synchronisation and a cudaFree
+// for every piece.)
 struct Scratch {
   unsigned char* base = nullptr;
   size_t bytes = 0;
@@ -416,11 +416,11 @@ size_t specx_count(const mrm_gpu* r) {
 int rows_per_task(const mrm_gpu* r, int rpb) { return r->wnx ? 1 : std::max(1, std::min(rpb, r->g.ny)); }
 
 // Runs whose column step is the register column kernel (colreg.cuh): FP32, one
-// layer with 64..1024-point columns or two with 512 or 1024 (shorter ones are
-// single runs whose blocks of six components crowd out the next kernel's early
-// start: 437 x 48 x 2 grains 54 us per step against 47 with the in-place kernel,
-// 500 x 75 x 2 60 against 54; 1024 x 256 x 2 190 against 235), with a symmetric
-// tensor (to kTensAsym of its largest value): that kernel keeps six components
+// layer with 64..1024-point columns or two with 512 or 1024 (in single runs of
+// shorter ones the blocks of six components crowd out the next kernel's early
+// start: 437 x 48 x 2 grains 54 us per step against 46 with the in-place kernel,
+// 500 x 75 x 2 60 against 54; 1024 x 256 x 2 190 against 235; batches of them
+// were not timed in both), with a symmetric tensor (to kTensAsym of its largest value): that kernel keeps six components
 // per layer pair (tensor.cuh pack_tensor_creg_kernel).  The SUL and head image
 // terms make N_xz and N_zx differ; such a tensor keeps its nine components and
 // the in-place column kernel, which also takes the other lengths and layer counts.
@@ -514,7 +514,7 @@ int run_stage_bytes(const mrm_gpu* r, int stage, int rows) {
 // task as the longest rows' tasks: its blocks then carry about as many points
 // as those of the longest rows instead of idling most of their threads.
 struct RowPackCap {
-  int fft = 0;     // FFT-buffer bytes of the launch (twiddles + two buffers)
+  int fft = 0;     // twiddles and FFT buffers of the launch (row_fft_smem), bytes
   int grains = 0;  // grains of the largest unpacked task
 };
 

@@ -196,9 +196,8 @@ MRM_D void reg_stage1(Cx<float>* b, int t, const Cx<float>* __restrict__ tw) {
 
 // Both transforms work in place in the sequence's one buffer: every stage's
 // loads are behind a barrier of the group before another thread's positions
-// are overwritten.  (A second buffer saved one barrier per transform and cost
-// half the resident blocks of the long rows: two 1024-point rows' blocks per
-// SM instead of four.)
+// are overwritten.  (A second buffer would save a barrier per transform and cost
+// half the resident blocks of the long rows.)
 
 // Inverse: b holds X (M + 1 spectrum values, natural order) -> z[n] for n < nz.
 // Thread t gathers the pre-processed spectrum at its first stage's positions,

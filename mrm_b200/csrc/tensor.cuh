@@ -107,9 +107,9 @@ __device__ __noinline__ TensCorner tens_corner(dd x, dd y, dd z) {
 // and three arctangents each).  T = 8: the 300 values of a tile and three
 // heights are two rounds of a 256-thread block, which is what a small grid's
 // few tiles wait for; T = 16 saves a fifth of the evaluations and doubles the rounds.
-// Measured against 64 evaluations per slot in one thread each: build_tensor with a
-// field evaluation on 512 x 512 slots 30.5 -> 1.66 ms, off_field on 1024 x 256 slots
-// and two layers 50.1 -> 2.65 ms (one call each, with its copies and allocation).
+// Measured with the calls' copies and allocation: build_tensor and a field
+// evaluation on 512 x 512 slots 1.7 to 2.4 ms (64 evaluations per slot: 30.5),
+// off_field on 1024 x 256 slots and two layers 2.7 to 3.5 ms (50.1).
 constexpr int kTensTile = 8, kTensBlock = 256, kTensItems = kTensTile * kTensTile * 6;
 MRM_HD constexpr int tens_rows(bool lattice_y) { return lattice_y ? kTensTile + 2 : 4 * kTensTile; }
 MRM_HD constexpr size_t tens_smem(bool lattice_y) {
