@@ -479,16 +479,16 @@ constexpr size_t kSmemPerSM = 228 * 1024;
 constexpr size_t kSmemReserved = 1024;  // per block
 
 // Shared memory that a row launch of `tasks` blocks asks for beyond what it uses,
-// beside the in-place column kernel of FP32 runs: just over a share of one more
-// block per SM than an even spread needs (at least two), so that no more fit.
-// Row blocks start while the column kernel's are still resident, wherever there
-// is room; with the 20 to 40 KB that they use, three or four go to one SM while
-// others have none, and the launch waits for those.  Two-layer runs, us per Heun
-// step without / with: 700 x 60 (120 blocks) 82.7 / 71.8, 537 x 120 (240) 105.2 /
-// 98.0, 600 x 200 (400) 152.9 / 139.0; 437 x 48 (96) 48.4 / 46.4, and 48.4 with
-// room for one.  Four per SM is what the registers hold anyway.  (A column launch
-// that leaves SMs empty is no obstacle: there the same asks for nothing, 64 x 64
-// grains 23.9 against 25.1.)
+// beside the column kernel of FP32 runs of two layers or of the in-place one: just
+// over a share of one more block per SM than an even spread needs (at least two),
+// so that no more fit.  Row blocks start while the column kernel's are still
+// resident, wherever there is room; with the 20 to 40 KB that they use, three or
+// four go to one SM while others have none, and the launch waits for those.
+// Two-layer runs, us per Heun step without / with: 700 x 60 (120 blocks) 82.7 /
+// 71.8, 537 x 120 (240) 105.2 / 98.0, 1000 x 140 (280) 156 / 138, 600 x 200 (400)
+// 151 / 140; 437 x 48 (96) 48.4 / 46.4, and 48.4 with room for one.  Four per SM is
+// what the registers hold anyway.  (A column launch that leaves SMs empty is no
+// obstacle: there the same asks for nothing, 64 x 64 grains 23.9 against 25.1.)
 size_t row_spread_smem(int tasks, int sms, size_t static_bytes) {
   const int per_sm = std::max(2, (tasks + sms - 1) / sms);
   return per_sm > 3 ? 0 : kSmemPerSM / (per_sm + 1) + 1024 - kSmemReserved - static_bytes;
@@ -771,6 +771,8 @@ int plan_smem(Engine* e) {
   size_t scol = 16;
   int tw_cap[2] = {0, 0}, stage_bytes[2] = {0, 0};
   const int cv[2] = {creg_v(e, 1), creg_v(e, 2)};
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
   const RowPackCap pack = row_pack_cap<R>(e, rv.rpb);
   for (auto* r : e->runs) {
     if (r->lgpx > rv.lgmax)
@@ -804,14 +806,17 @@ int plan_smem(Engine* e) {
   if (scol + 64 > kMaxSmem) return set_err(errp, MRM_ERR_UNSUPPORTED, "column shape exceeds shared memory");
   e->smem_col = scol;
   for (int i = 0; i < 2; ++i) {
-    const size_t screg = tw_cap[i] ? creg_smem_of(cv[i], i + 1, tw_cap[i], stage_bytes[i]) : 16;
+    size_t screg = tw_cap[i] ? creg_smem_of(cv[i], i + 1, tw_cap[i], stage_bytes[i]) : 16;
+    // two layers, no more tasks than SMs: one block to an SM, by the same reasoning
+    // as row_spread_smem (two of them started early on one SM take turns: 200 x
+    // 250 x 2 grains 60.4 us per Heun step, 52.0 with one; 100 x 200 x 2 57.4, 47.4)
+    if (i == 1 && tw_cap[i] && e->nct2[i] <= sms)
+      screg = std::max(screg, kSmemPerSM / 2 + 1024 - kSmemReserved - kCregStatic);
     if (screg + kCregStatic > kMaxSmem) return set_err(errp, MRM_ERR_UNSUPPORTED, "column shape exceeds shared memory");
     e->smem_creg[i] = screg;
     e->creg_tw_cap[i] = tw_cap[i];
   }
-  int sms = 0;
-  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev));
-  const bool spread = sizeof(R) == sizeof(float) && e->nct >= sms && !e->nct2[0] && !e->nct2[1];
+  const bool spread = sizeof(R) == sizeof(float) && std::max(e->nct, e->nct2[1]) >= sms && !e->nct2[0];
   if (spread)
     for (int q = 0; q < kSlots; ++q)
       e->smem_row[q] = std::max(e->smem_row[q], row_spread_smem(e->nrt, sms, row_static_bytes(q)));

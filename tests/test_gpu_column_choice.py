@@ -132,3 +132,23 @@ def test_column_shape_without_the_tuner(gpulib):
         g.step(8, 1e-13)
         assert g.get_shape()[1] == col
         g.close()
+
+
+@pytest.mark.parametrize("nx,ny,row,col", [(200, 250, 4, 1), (40, 500, 4, 1), (600, 200, 3, 2), (1000, 140, 2, 2)])
+def test_blocks_of_two_layer_runs_spread_over_the_sms(gpulib, nx, ny, row, col):
+    """Two-layer runs on the register column kernel: one column block to an SM where
+    there are no more tasks than SMs; row blocks as for the in-place kernel."""
+    med = media.two_layer_medium(nx, ny, seed=4, temperature=300.0)
+    b = Batch(FP32)
+    r = b.add(med, dt=1e-13, steps=10, thermal_seed=3)
+    r.set_shape(0, 1, 1)
+    b.step(10)
+    b.stats([r])
+    assert b.occupancy() == (row, col)
+    g = GpuSim(med, precision=FP32, thermal_seed=3)
+    g.set_shape(1, 0, 1)
+    g.step(10, 1e-13)
+    for l in range(2):
+        assert np.array_equal(r.get_state(l), g.get_state(l))
+    g.close()
+    b.close()
